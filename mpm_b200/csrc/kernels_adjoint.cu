@@ -86,7 +86,7 @@ __device__ __forceinline__ void box_point(const DevState& s, int c, const double
   int ijk[3] = {0, 0, 0};
   cell_ijk<DIM>(s, c, ijk);
 #pragma unroll
-  for (int d = 0; d < DIM; ++d) b.ihl[d] = s.axis_ihl[d][ijk[d]];
+  for (int d = 0; d < DIM; ++d) b.ihl[d] = s.axcell[d][ijk[d]].ihl;
   grid_cell_nodes<DIM>(s, c, b.nid);
 }
 
@@ -454,7 +454,7 @@ __global__ void __launch_bounds__(256) k_adj_scatter(DevState s, AdjointArgs A) 
     cell_ijk<DIM>(s, (int)c, ijk);
 #pragma unroll
     for (int d = 0; d < DIM; ++d) {
-      ihl[d] = s.axis_ihl[d][ijk[d]];
+      ihl[d] = s.axcell[d][ijk[d]].ihl;
       dc[d] = s.dndx_c[((int64_t)c * NV + k) * DIM + d];
     }
   }

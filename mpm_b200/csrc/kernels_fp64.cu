@@ -745,7 +745,7 @@ __global__ void __launch_bounds__(128, MPM_G2P_MIN_BLOCKS) k_g2p(DevState s, dou
     s.lost[atomicAdd(s.nlost, 1u)] = (int32_t)p;
     return;
   }
-  const int nc = locate_near<DIM>(s, xn, c);
+  const int nc = locate_near<DIM, BOX>(s, xn, c);
   if (nc >= 0) {
     if (nc != c) s.cell[p] = nc;
   } else {
@@ -899,7 +899,7 @@ __global__ void __launch_bounds__(STAGE_T, MPM_G2P_MIN_BLOCKS)
       raise_err(s, ERR_NONFINITE);
       s.lost[atomicAdd(s.nlost, 1u)] = (int32_t)p;
     } else {
-      const int nc = locate_near<DIM>(s, xn, c);
+      const int nc = locate_near<DIM, BOX>(s, xn, c);
       if (nc >= 0) {
         if (nc != c) s.cell[p] = nc;
       } else {
@@ -971,7 +971,7 @@ __global__ void __launch_bounds__(128, MPM_G2P_MIN_BLOCKS) k_g2p_musl(DevState s
 }
 
 // MUSL end of step: the new positions replace the old, then locate
-template <int DIM>
+template <int DIM, bool BOX>
 __global__ void __launch_bounds__(128) k_commit_locate(DevState s) {
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= s.np) return;
@@ -991,7 +991,7 @@ __global__ void __launch_bounds__(128) k_commit_locate(DevState s) {
     s.lost[atomicAdd(s.nlost, 1u)] = (int32_t)p;
     return;
   }
-  const int nc = locate_near<DIM>(s, xn, c);
+  const int nc = locate_near<DIM, BOX>(s, xn, c);
   if (nc >= 0) {
     if (nc != c) s.cell[p] = nc;
   } else {
@@ -1141,7 +1141,7 @@ void step_impl(const DevState& s, const StepArgs& a, cudaStream_t st, Profiler& 
     pr.end(K_STRESS, st);
     mc_returns();
     pr.begin(K_LOCATE, st);
-    k_commit_locate<DIM><<<pb128, 128, 0, st>>>(s);
+    k_commit_locate<DIM, BOX><<<pb128, 128, 0, st>>>(s);
     pr.end(K_LOCATE, st);
   } else if (a.scheme == 1) {  // USL
     pr.begin(K_P2G, st);

@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(tangent_tile_t<BOX>(), MPM_TANGENT_P2G_MIN_BLO
     int ijk[3] = {0, 0, 0};
     if (a1 > a0) cell_ijk<DIM>(s, (int)c, ijk);
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) ihl[d] = a1 > a0 ? s.axis_ihl[d][ijk[d]] : 0.;
+    for (int d = 0; d < DIM; ++d) ihl[d] = a1 > a0 ? s.axcell[d][ijk[d]].ihl : 0.;
   }
   const double gv[3] = {g0, g1, g2};
   const int64_t np = s.np;
@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(128, MPM_TANGENT_G2P_MIN_BLOCKS) k_stress_tang
     int ijk[3] = {0, 0, 0};
     cell_ijk<DIM>(s, c, ijk);
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) ihl[d] = s.axis_ihl[d][ijk[d]];
+    for (int d = 0; d < DIM; ++d) ihl[d] = s.axcell[d][ijk[d]].ihl;
   } else {
     jinv_dual<DIM>(xi, X, inv);
   }
@@ -595,7 +595,7 @@ __global__ void __launch_bounds__(128, MPM_TANGENT_KIN_MIN_BLOCKS) k_g2p_tangent
     s.lost[atomicAdd(s.nlost, 1u)] = (int32_t)p;
     return;
   }
-  const int nc = locate_near<DIM>(s, xn, c);
+  const int nc = s.structured ? locate_near<DIM, true>(s, xn, c) : locate_near<DIM, false>(s, xn, c);
   if (nc >= 0) {
     if (nc != c) s.cell[p] = nc;
   } else {

@@ -114,16 +114,20 @@ __device__ __forceinline__ void load_x(const DevState& s, int64_t p, double* x) 
   for (int d = 0; d < DIM; ++d) x[d] = s.pf[(int64_t)(PF<DIM>::X + d) * s.np + p];
 }
 
+// n / f.d for 0 <= n < 2^31
+__device__ __forceinline__ int fast_div(const FastDiv& f, int n) {
+  return (int)((__umulhi(f.mul, (unsigned)n) + (unsigned)n) >> f.shift);
+}
+
 // cell (i, j, k) of a tensor-product grid
 template <int DIM>
 __device__ __forceinline__ void cell_ijk(const DevState& s, int c, int* ijk) {
-  ijk[0] = c % s.gcells[0];
-  if constexpr (DIM == 2) {
-    ijk[1] = c / s.gcells[0];
-  } else {
-    ijk[1] = (c / s.gcells[0]) % s.gcells[1];
-    ijk[2] = c / (s.gcells[0] * s.gcells[1]);
+  if constexpr (DIM == 3) {
+    ijk[2] = fast_div(s.div_gxy, c);
+    c -= ijk[2] * (int)s.div_gxy.d;
   }
+  ijk[1] = fast_div(s.div_gx, c);
+  ijk[0] = c - ijk[1] * s.gcells[0];
 }
 
 // local node n of a cell -> offset (di, dj, dk) (quadrilateral_element.tcc:1-7,
@@ -158,10 +162,11 @@ __device__ __forceinline__ void grid_node_cells(const DevState& s, int node, int
                                                 int* count) {
   constexpr int NC = DIM == 2 ? 4 : 8;
   const int gx = s.gcells[0], gy = s.gcells[1], gz = s.gcells[2];
-  const int nx = gx + 1, ny = gy + 1;
-  const int i = node % nx;
-  const int j = DIM == 2 ? node / nx : (node / nx) % ny;
-  const int k = DIM == 2 ? 0 : node / (nx * ny);
+  const int nx = gx + 1;
+  const int k = DIM == 2 ? 0 : fast_div(s.div_nxy, node);
+  const int in_layer = DIM == 2 ? node : node - k * (int)s.div_nxy.d;
+  const int j = fast_div(s.div_nx, in_layer);
+  const int i = in_layer - j * nx;
 #pragma unroll
   for (int q = 0; q < NC; ++q) {
     const int a = q & 1, b = (q >> 1) & 1, e = q >> 2;  // cell (i - 1 + a, j - 1 + b, k - 1 + e)
@@ -272,7 +277,7 @@ __device__ __forceinline__ CellMap<DIM, BOX, R> cell_map(const DevState& s, int 
     int ijk[3] = {0, 0, 0};
     cell_ijk<DIM>(s, c, ijk);
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) m.ihl[d] = R(__ldg(&s.axis_ihl[d][ijk[d]]));
+    for (int d = 0; d < DIM; ++d) m.ihl[d] = R(__ldg(&s.axcell[d][ijk[d]].ihl));
   } else {
     jacobian_inverse<DIM>(xi, X, m.inv);
   }
@@ -448,6 +453,32 @@ __device__ __forceinline__ bool cell_point_in(const DevState& s, int c, const do
   return point_in_cell<DIM>(x, g.centroid, g.len, g.mean_length, xi);
 }
 
+// a / b from r = the rounded 1 / b: the product a r corrected by its exact
+// remainder (Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990).  Three operations; the quotient is a / b
+// rounded once unless a / b lies within 2^-104 of itself of a rounding
+// boundary.
+__device__ __forceinline__ double quotient_by(double a, double b, double r) {
+  const double q = a * r;
+  return fma(fma(-b, q, a), r, q);
+}
+
+// local_xi in cell ijk of a tensor-product grid, from the axis tables: a few
+// hundred records that stay in L1, where a warp's cells would read 56 bytes
+// each from the per-cell table.
+template <int DIM>
+__device__ __forceinline__ void box_xi(const DevState& s, const int* ijk, const double* x,
+                                       double* xi) {
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) {
+    const AxisCell g = s.axcell[d][ijk[d]];
+    double v = quotient_by(2. * (x[d] - g.centroid), g.len, g.rlen);
+    if (v < -1. + kDblEps) v = -1. + kDblEps;
+    if (v > 1. - kDblEps) v = 1. - kDblEps;
+    xi[d] = v;
+  }
+}
+
 // Local coordinates of a particle at x in the cell it was last located in,
 // bit-identical to the value the locate step found (same function, same
 // inputs): the Cartesian formula on box cells and without s.iso, else the
@@ -455,8 +486,12 @@ __device__ __forceinline__ bool cell_point_in(const DevState& s, int c, const do
 template <int DIM, bool BOX>
 __device__ __forceinline__ void particle_xi(const DevState& s, int c, const double* x,
                                             double* xi) {
-  const CellGeom& g = s.geom[c];
-  if constexpr (!BOX) {
+  if constexpr (BOX) {
+    int ijk[3] = {0, 0, 0};
+    cell_ijk<DIM>(s, c, ijk);
+    box_xi<DIM>(s, ijk, x, xi);
+  } else {
+    const CellGeom& g = s.geom[c];
     if (s.iso) {
       constexpr int NV = Elem<DIM>::NV;
       int nid[NV];
@@ -470,41 +505,72 @@ __device__ __forceinline__ void particle_xi(const DevState& s, int c, const doub
       }
       return;
     }
+    local_xi<DIM>(x, g.centroid, g.len, xi);
   }
-  local_xi<DIM>(x, g.centroid, g.len, xi);
 }
 
-// mesh.tcc:1116-1151: the current cell, then neighbours in ascending id
+// Whether x lies in axis interval i of a tensor-product grid, as point_in_cell
+// decides it for a cell over that interval: |2 (x - centroid) / len| <= 1.
+// The rounded quotient exceeds 1 exactly when its numerator exceeds len (the
+// smallest such quotient, 1 + ulp(len) / len, is more than half an ulp above
+// 1), so no division is needed; NaN is outside.
+__device__ __forceinline__ bool in_interval(const AxisCell* ax, int i, double x) {
+  return fabs(2. * (x - ax[i].centroid)) <= ax[i].len;
+}
+
+// The locate of a tensor-product grid from cell c at ijk: c if it holds x,
+// else the first of the 3^dim - 1 cells around it in ascending id (the
+// node-sharing cells of mesh.tcc:287-306), or -1.  A cell holds x when each of
+// its axis intervals does, and ids ascend with (k, j, i), so the first cell is
+// the first interval per axis.  point_in_cell's distance test never decides:
+// a point of a box is within (a + b + c) / 2 of its centroid, 1.5 mean edge
+// lengths (1 in 2D), and the test allows 2.
 template <int DIM>
-__device__ __forceinline__ int locate_near(const DevState& s, const double* x, int c) {
+__device__ __forceinline__ int locate_box(const DevState& s, const double* x, int c,
+                                          const int* ijk) {
+  bool here = true;
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) here = here && in_interval(s.axcell[d], ijk[d], x[d]);
+  if (here) return c;
+  int to[3] = {0, 0, 0};
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) {
+    const int lo = ijk[d] > 0 ? ijk[d] - 1 : 0;
+    const int hi = ijk[d] + 1 < s.gcells[d] ? ijk[d] + 1 : ijk[d];
+    int i = lo;
+    while (i <= hi && !in_interval(s.axcell[d], i, x[d])) ++i;
+    if (i > hi) return -1;
+    to[d] = i;
+  }
+  return DIM == 2 ? to[0] + s.gcells[0] * to[1] : to[0] + s.gcells[0] * (to[1] + s.gcells[1] * to[2]);
+}
+
+// the search of a general mesh over its neighbour lists
+template <int DIM>
+__device__ __forceinline__ int locate_general(const DevState& s, const double* x, int c) {
   double xi[DIM];
   if (cell_point_in<DIM>(s, c, x, xi)) return c;
-  if (s.structured) {
-    // neighbours of a tensor-product cell: the 3^dim - 1 cells around it,
-    // ascending id (the node-sharing cells of mesh.tcc:287-306)
-    int ijk[3] = {0, 0, 0};
-    cell_ijk<DIM>(s, c, ijk);
-    const int kmin = DIM == 3 ? ijk[2] - 1 : 0, kmax = DIM == 3 ? ijk[2] + 1 : 0;
-    for (int k = kmin; k <= kmax; ++k) {
-      if (DIM == 3 && (k < 0 || k >= s.gcells[2])) continue;
-      for (int j = ijk[1] - 1; j <= ijk[1] + 1; ++j) {
-        if (j < 0 || j >= s.gcells[1]) continue;
-        for (int i = ijk[0] - 1; i <= ijk[0] + 1; ++i) {
-          if (i < 0 || i >= s.gcells[0]) continue;
-          const int nc = DIM == 2 ? i + s.gcells[0] * j : i + s.gcells[0] * (j + s.gcells[1] * k);
-          if (nc == c) continue;
-          if (cell_point_in<DIM>(s, nc, x, xi)) return nc;
-        }
-      }
-    }
-    return -1;
-  }
   const int b = s.nb_off[c], e = s.nb_off[c + 1];
   for (int k = b; k < e; ++k) {
     const int nc = s.nb[k];
     if (cell_point_in<DIM>(s, nc, x, xi)) return nc;
   }
   return -1;
+}
+
+// mesh.tcc:1116-1151: the current cell, then neighbours in ascending id.  BOX
+// (a tensor-product grid) is a template argument, since the general search's
+// isoparametric map would take registers in every kernel that holds it: the
+// staged mixed G2P spilled 470 bytes a thread for it at 80 registers.
+template <int DIM, bool BOX>
+__device__ __forceinline__ int locate_near(const DevState& s, const double* x, int c) {
+  if constexpr (BOX) {
+    int ijk[3] = {0, 0, 0};
+    cell_ijk<DIM>(s, c, ijk);
+    return locate_box<DIM>(s, x, c, ijk);
+  } else {
+    return locate_general<DIM>(s, x, c);
+  }
 }
 
 

@@ -325,7 +325,7 @@ struct mpm_gpu_solver {
   bool isoparametric = false;  // general cells: isoparametric local coordinates
   int32_t gcells[3] = {1, 1, 1};
   std::vector<double> axis[3];
-  std::vector<double> axis_ihl[3];  // 2 / (axis[i + 1] - axis[i]): J^-1 of the box cells
+  std::vector<AxisCell> axcell[3];  // the cells' geometry per axis interval
 
   // materials
   std::vector<MaterialParams> mats;
@@ -357,7 +357,7 @@ struct mpm_gpu_solver {
   DevBuf<uint8_t> d_rpass;
   DevBuf<MaterialParams> d_mats;
   DevBuf<double> d_axis[3];
-  DevBuf<double> d_axis_ihl[3];
+  DevBuf<AxisCell> d_axcell[3];
   DevBuf<double> d_dndx_c, d_partials;
   DevBuf<int32_t> d_nc_off, d_nc_cell, d_cnt, d_start, d_rank, d_order, d_bsum;
   DevBuf<int8_t> d_nc_slot;
@@ -620,8 +620,12 @@ bool detect_structured(mpm_gpu_t h) {
   for (int d = 0; d < 3; ++d) {
     h->axis[d] = d < dim ? ax[d] : std::vector<double>{0.0, 1.0};
     const std::vector<double>& a = h->axis[d];
-    h->axis_ihl[d].resize(a.size() - 1);
-    for (size_t i = 0; i + 1 < a.size(); ++i) h->axis_ihl[d][i] = 2. / (a[i + 1] - a[i]);
+    h->axcell[d].resize(a.size() - 1);
+    const int64_t step = d == 0 ? 1 : (d == 1 ? cx : cx * cy);
+    for (size_t i = 0; i + 1 < a.size(); ++i) {
+      const CellGeom g = d < dim ? h->geom[i * step] : CellGeom{{0.5, 0.5, 0.5}, {1., 1., 1.}, 1.};
+      h->axcell[d][i] = AxisCell{g.centroid[d], g.len[d], 1. / g.len[d], 2. / (a[i + 1] - a[i])};
+    }
   }
   return true;
 }
@@ -759,7 +763,7 @@ void upload_mesh(mpm_gpu_t h) {
   if (h->structured)
     for (int d = 0; d < 3; ++d) {
       h->d_axis[d].upload(h->axis[d].data(), h->axis[d].size(), st);
-      h->d_axis_ihl[d].upload(h->axis_ihl[d].data(), h->axis_ihl[d].size(), st);
+      h->d_axcell[d].upload(h->axcell[d].data(), h->axcell[d].size(), st);
     }
   if (h->mixed) {
     std::vector<float> f(h->dndx_c.begin(), h->dndx_c.end());
@@ -937,8 +941,12 @@ void refresh_state(mpm_gpu_t h) {
   for (int d = 0; d < 3; ++d) {
     s.gcells[d] = h->gcells[d];
     s.axis[d] = h->d_axis[d].p;
-    s.axis_ihl[d] = h->d_axis_ihl[d].p;
+    s.axcell[d] = h->d_axcell[d].p;
   }
+  s.div_gx = make_fast_div((uint32_t)h->gcells[0]);
+  s.div_gxy = make_fast_div((uint32_t)(h->gcells[0] * (int64_t)h->gcells[1]));
+  s.div_nx = make_fast_div((uint32_t)(h->gcells[0] + 1));
+  s.div_nxy = make_fast_div((uint32_t)((h->gcells[0] + 1) * (int64_t)(h->gcells[1] + 1)));
   s.nc_off = h->d_nc_off.p;
   s.nc_cell = h->d_nc_cell.p;
   s.nc_slot = h->d_nc_slot.p;

@@ -76,6 +76,27 @@ struct ParticleVC {
   double value[3];
 };
 
+// One interval of a tensor-product grid's axis: the centroid and length that
+// CellGeom holds for every cell over it (bit for bit), 1 / len and 2 / the
+// difference of the axis coordinates (J^-1 of a box cell).
+struct alignas(32) AxisCell {
+  double centroid, len, rlen, ihl;
+};
+
+// Division of ids below 2^31 by a fixed divisor as a high product and a shift
+// (Granlund and Montgomery, "Division by invariant integers using
+// multiplication", 1994, figure 4.1, whose sum cannot overflow for n < 2^31).
+struct FastDiv {
+  uint32_t d = 1, mul = 1, shift = 0;
+};
+inline FastDiv make_fast_div(uint32_t d) {
+  FastDiv f;
+  f.d = d;
+  while ((1ull << f.shift) < d) ++f.shift;
+  f.mul = (uint32_t)((((1ull << f.shift) - d) << 32) / d + 1);
+  return f;
+}
+
 enum ErrorBits : unsigned {
   ERR_OUTSIDE = 1u,     // a particle left the mesh (locate_particles on)
   ERR_NONFINITE = 2u,   // NaN or Inf in a particle position
@@ -117,7 +138,9 @@ struct DevState {
   int structured = 0;
   int32_t gcells[3] = {1, 1, 1};     // cells per axis
   const double* axis[3] = {nullptr, nullptr, nullptr};  // node coordinates per axis
-  const double* axis_ihl[3] = {nullptr, nullptr, nullptr};  // 2 / cell length per axis interval
+  const AxisCell* axcell[3] = {nullptr, nullptr, nullptr};  // per axis interval
+  FastDiv div_gx, div_gxy;           // cells per row and per layer
+  FastDiv div_nx, div_nxy;           // nodes per row and per layer
   double* mapb = nullptr;  // [DIM * DIM][np] mapping matrix (ASFLIP, TPIC, APIC), row-major
   int iso = 0;             // general cells take isoparametric local coordinates
 

@@ -1,0 +1,58 @@
+"""Tensor-product grids with graded axes: the box-cell kernels (axis tables, the
+division-free locate, interpolation along the axes) against the CPU oracle, which
+knows cells only by their nodes, and mixed against FP64.
+
+Every other grid of the tests is uniform and cubic; here each axis has its own
+spacings, the cell counts are odd and differ per axis, and the particles move
+across cells.
+"""
+import numpy as np
+import pytest
+
+from mpm_b200 import problems as P
+from oracle.oracle import build_oracle
+from tests.parity import assert_parity, field_errors
+
+pytestmark = pytest.mark.gpu
+
+
+def graded(dim, scheme, update="flip"):
+    """A linear elastic block flying through a graded grid."""
+    shape = (13, 9) if dim == 2 else (11, 7, 5)
+    if dim == 2:
+        prob = P.column_2d(shape=shape, block=(5, 4), E=5e5, scheme=scheme, dt=1e-4, velocity_update=update)
+    else:
+        prob = P.column_3d(shape=shape, block=(4, 3, 3), material="LinearElastic", E=5e5, scheme=scheme, dt=1e-4,
+                           geostatic=False, velocity_update=update)
+    rng = np.random.default_rng(5)
+    axes = [np.concatenate([[0.0], np.cumsum(prob.dx * rng.uniform(0.6, 1.7, n))]) for n in shape]
+    old = [np.arange(n + 1) * prob.dx for n in shape]
+    stretch = lambda x: np.stack([np.interp(x[:, d], old[d], axes[d]) for d in range(dim)], axis=1)  # noqa: E731
+    prob.coords = np.stack([axes[d][np.rint(prob.coords[:, d] / prob.dx).astype(int)] for d in range(dim)], axis=1)
+    prob.particles = [(stretch(p), m) for p, m in prob.particles]
+    return prob
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("scheme,update", [("usl", "flip"), ("usf", "pic"), ("musl", "flip"), ("usl", "apic")])
+def test_graded_grid(dim, scheme, update):
+    prob = graded(dim, scheme, update)
+    g, m, o = (P.build_solver(prob), P.build_solver(prob, precision="mixed"), build_oracle(prob))
+    st = g.read()
+    v = np.tile(np.array([0.9, 0.4, 0.3])[:dim], (len(st["x"]), 1))
+    st["v"] = v
+    g.load(st)
+    m.load(st)
+    so = o.get()
+    so["v"][:, :dim] = v
+    o.set(so)
+    start = st["cell"].copy()
+    for n in (1, 99):
+        for s in (g, m, o):
+            s.step(n)
+        a, b = g.read(), o.get()
+        assert_parity(a, b, label=f"{dim}D {scheme} {update}")
+    assert np.count_nonzero(a["cell"] != start) > len(start) // 4, "the block was meant to cross cells"
+    errs = field_errors(m.read(), a)
+    # FP32 increments of 100 steps: each adds at most a few 2^-24 of the field's scale
+    assert max(errs.values()) < 100 * 4 * 2.0 ** -24, errs
