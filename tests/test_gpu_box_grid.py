@@ -17,7 +17,7 @@ pytestmark = pytest.mark.gpu
 
 
 def graded(dim, scheme, update="flip"):
-    """A linear elastic block flying through a graded grid."""
+    """A free linear elastic block flying through a graded grid."""
     shape = (13, 9) if dim == 2 else (11, 7, 5)
     if dim == 2:
         prob = P.column_2d(shape=shape, block=(5, 4), E=5e5, scheme=scheme, dt=1e-4, velocity_update=update)
@@ -29,8 +29,17 @@ def graded(dim, scheme, update="flip"):
     old = [np.arange(n + 1) * prob.dx for n in shape]
     stretch = lambda x: np.stack([np.interp(x[:, d], old[d], axes[d]) for d in range(dim)], axis=1)  # noqa: E731
     prob.coords = np.stack([axes[d][np.rint(prob.coords[:, d] / prob.dx).astype(int)] for d in range(dim)], axis=1)
-    prob.particles = [(stretch(p), m) for p, m in prob.particles]
+    prob.particles = [(stretch(p + prob.dx), m) for p, m in prob.particles]
+    prob.velocity_constraints = prob.friction_constraints = None
+    prob.analysis["gravity"] = (0.0,) * dim
     return prob
+
+
+def start_velocity(x):
+    """Translation and a linear field (spin and stretch)."""
+    dim = x.shape[1]
+    grad = np.array([[0.5, 2.0, -1.0], [-1.5, -0.8, 0.7], [1.0, -0.6, 0.4]])[:dim, :dim]
+    return np.array([0.9, 0.5, 0.4])[:dim] + x @ grad.T
 
 
 @pytest.mark.parametrize("dim", [2, 3])
@@ -39,8 +48,7 @@ def test_graded_grid(dim, scheme, update):
     prob = graded(dim, scheme, update)
     g, m, o = (P.build_solver(prob), P.build_solver(prob, precision="mixed"), build_oracle(prob))
     st = g.read()
-    v = np.tile(np.array([0.9, 0.4, 0.3])[:dim], (len(st["x"]), 1))
-    st["v"] = v
+    st["v"] = v = start_velocity(st["x"])
     g.load(st)
     m.load(st)
     so = o.get()
