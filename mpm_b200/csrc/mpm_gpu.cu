@@ -721,6 +721,7 @@ MaterialParams make_material(int dim, const std::string& type, const Json& j) {
     m.cos_phi = std::cos(m.phi_peak);
     m.tan_phi = std::tan(m.phi_peak);
     m.tan_psi = std::tan(m.psi_peak);
+    friction_quotients(m.sin_phi, m.cos_phi, m.ic_phi, m.e_phi, m.n_phi);
   } else {
     throw InvalidArg("unknown material type \"" + type + "\"");
   }

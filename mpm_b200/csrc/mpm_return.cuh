@@ -89,7 +89,7 @@ __device__ __forceinline__ bool mc_begin(const MaterialT<R>& m, const R* stress,
 // The trial stress's dF/dsigma is needed only when the old stress is off the
 // yield surface; mc_stress keeps the trial invariants for it, here the pass
 // MR_TRIAL_DF evaluates them again (the same inputs give the same values)
-// into q.sv, which changes only epsilon, rho and theta there -- evaluated again
+// into q.sv, which changes only epsilon and rho there -- evaluated again
 // at the corrected stress before anything else reads them.
 template <typename R>
 __device__ __forceinline__ bool mc_pass(const MaterialT<R>& m, const R* stress, const R* dstrain,
@@ -181,6 +181,7 @@ __device__ __forceinline__ void mc_return(const MaterialT<R>& m, const R* stress
   if (!mc_begin(m, stress, dstrain, density, q, out)) {
     while (!mc_pass(m, stress, dstrain, q, out)) {
     }
+    q.sv[SV_THETA] = mc_lode_angle(q.lt);  // of the last pass's stress, the final one
   }
 #pragma unroll
   for (int k = 0; k < SV_N; ++k) sv[k] = q.sv[k];
