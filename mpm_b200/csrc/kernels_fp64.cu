@@ -21,6 +21,7 @@
 #include "mpm_bulk.cuh"
 #include "mpm_device.cuh"
 #include "mpm_kernels.h"
+#include "mpm_launch.cuh"
 #include "mpm_return.cuh"
 #include "mpm_state.cuh"
 
@@ -41,22 +42,23 @@ namespace mpm_b200 {
 namespace {
 
 // ------------------------------------------------------------ counting sort
+// The counts (and, with words, the step's list lengths) set to zero.
+__global__ void __launch_bounds__(256) k_sort_reset(DevState s, int words) {
+  after_previous();
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < s.ncells;
+       i += (int64_t)gridDim.x * blockDim.x)
+    s.cnt[i] = 0;
+  if (words && blockIdx.x == 0 && threadIdx.x == 0) *s.nlost = *s.nplastic = *s.nplastic_heavy = 0;
+}
+
 __global__ void __launch_bounds__(256) k_count(DevState s) {
+  after_previous();
   count_particle(s, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
-// exclusive scan of n ints, SCAN_BLOCK per block (1024 threads x 4)
-__global__ void __launch_bounds__(1024) k_scan_local(const int32_t* in, int32_t* out,
-                                                     int32_t* bsum, int64_t n) {
-  __shared__ int32_t warp_tot[32];
-  const int64_t base = (int64_t)blockIdx.x * SCAN_BLOCK + threadIdx.x * 4;
-  int32_t v[4], e[4], t = 0;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    v[i] = (base + i < n) ? in[base + i] : 0;
-    e[i] = t;
-    t += v[i];
-  }
+// Exclusive sums of the block's per-thread totals t (1024 threads); *all
+// receives the block's total.
+__device__ __forceinline__ int32_t block_exclusive_sum(int32_t t, int32_t* warp_tot, int32_t* all) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   int32_t x = t;
 #pragma unroll
@@ -76,23 +78,86 @@ __global__ void __launch_bounds__(1024) k_scan_local(const int32_t* in, int32_t*
     warp_tot[lane] = z;
   }
   __syncthreads();
-  const int32_t prefix = (w > 0 ? warp_tot[w - 1] : 0) + x - t;
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-    if (base + i < n) out[base + i] = prefix + e[i];
-  if (threadIdx.x == 1023 && bsum) bsum[blockIdx.x] = prefix + t;
+  *all = warp_tot[31];
+  return (w > 0 ? warp_tot[w - 1] : 0) + x - t;
 }
 
-// add the scanned block totals; start[n] = total
-__global__ void __launch_bounds__(256) k_scan_add(int32_t* out, const int32_t* bscan,
-                                                  const int32_t* bsum, int64_t n, int64_t nb) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] += bscan[i / SCAN_BLOCK];
-  if (i == 0) out[n] = bscan[nb - 1] + bsum[nb - 1];
+// exclusive scan of the counts within chunks of SCAN_BLOCK cells, one per
+// block (1024 threads x 4), and the chunks' totals
+__global__ void __launch_bounds__(1024) k_scan_local(DevState s) {
+  __shared__ int32_t warp_tot[32];
+  after_previous();
+  const int64_t n = s.ncells, base = (int64_t)blockIdx.x * SCAN_BLOCK + threadIdx.x * 4;
+  int32_t v[4], e[4], t = 0, all;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    v[i] = (base + i < n) ? s.cnt[base + i] : 0;
+    e[i] = t;
+    t += v[i];
+  }
+  const int32_t prefix = block_exclusive_sum(t, warp_tot, &all);
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    if (base + i < n) s.start[base + i] = prefix + e[i];
+  if (threadIdx.x == 0) s.bsum[blockIdx.x] = all;
+}
+
+// Each chunk's starts plus the total of the chunks before it, which the block
+// adds up itself (at most SCAN_BLOCK totals; a kernel that scanned them first
+// would be one more dependent launch); start[n] = total.
+__global__ void __launch_bounds__(1024) k_scan_add(DevState s) {
+  __shared__ int32_t warp_tot[32];
+  after_previous();
+  int32_t t = 0, prefix;
+  for (int j = threadIdx.x; j < (int)blockIdx.x; j += 1024) t += s.bsum[j];
+  block_exclusive_sum(t, warp_tot, &prefix);
+  const int64_t n = s.ncells, base = (int64_t)blockIdx.x * SCAN_BLOCK;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int64_t c = base + i * 1024 + threadIdx.x;
+    if (c < n) s.start[c] += prefix;
+  }
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) s.start[n] = prefix + s.bsum[blockIdx.x];
 }
 
 __global__ void __launch_bounds__(256) k_fill(DevState s) {
+  after_previous();
   fill_particle(s, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
+}
+
+// The whole sort of a small problem in one cluster of SORT_CLUSTER blocks: its
+// passes are a few microseconds of dependent loads each, so the launches
+// between them cost more than the work; a cluster barrier takes well under
+// one.
+constexpr int SORT_CLUSTER = 8;
+__global__ void __cluster_dims__(SORT_CLUSTER, 1, 1) __launch_bounds__(1024) k_sort_small(DevState s, int words) {
+  namespace cg = cooperative_groups;
+  __shared__ int32_t warp_tot[32], totals[SORT_CLUSTER];
+  constexpr int NT = SORT_CLUSTER * 1024;
+  cg::cluster_group cl = cg::this_cluster();
+  after_previous();
+  const int r = (int)blockIdx.x, first = r * 1024 + (int)threadIdx.x;
+  const int nc = (int)s.ncells, np = (int)s.np;
+  for (int i = first; i < nc; i += NT) s.cnt[i] = 0;
+  if (words && first == 0) *s.nlost = *s.nplastic = *s.nplastic_heavy = 0;
+  cl.sync();
+  for (int p = first; p - (int)(threadIdx.x & 31) < np; p += NT) count_particle(s, p);  // whole warps
+  cl.sync();
+  // block r scans the r-th run of cells, each thread a run of it
+  const int per = (nc + NT - 1) / NT, c0 = min(nc, first * per), c1 = min(nc, c0 + per);
+  int32_t t = 0, all;
+  for (int c = c0; c < c1; ++c) t += s.cnt[c];
+  int32_t prefix = block_exclusive_sum(t, warp_tot, &all);
+  if (threadIdx.x < SORT_CLUSTER) *cl.map_shared_rank(&totals[r], threadIdx.x) = all;
+  cl.sync();
+  for (int q = 0; q < r; ++q) prefix += totals[q];
+  for (int c = c0; c < c1; ++c) {
+    s.start[c] = prefix;
+    prefix += s.cnt[c];
+  }
+  if (first == NT - 1) s.start[nc] = prefix;
+  cl.sync();
+  for (int p = first; p < np; p += NT) fill_particle(s, p);
 }
 
 // ---------------------------------------------------------------- P2G tiles
@@ -137,6 +202,7 @@ constexpr int tile_min_blocks() {
 template <int DIM, int MODE, bool BOX, int AFF, int T = p2g_tile_t<BOX, AFF>()>
 __global__ void __launch_bounds__(T, (tile_min_blocks<BOX, AFF, T>()))
     k_p2g_tiles(DevState s, double g0, double g1, double g2) {
+  after_previous();
   constexpr int NV = Elem<DIM>::NV;
   constexpr int CB = T / NV;
   constexpr int NVAL = PV<DIM>::N;
@@ -362,6 +428,7 @@ __device__ __forceinline__ void node_accel_update(const DevState& s, double m, c
 // 2: acceleration update on the velocity of the first pass (USF)
 template <int DIM, int MODE>
 __global__ void __launch_bounds__(256) k_nodes(DevState s, double dt, double damping) {
+  after_previous();
   const int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= s.nn) return;
   const int64_t nn = s.nn;
@@ -578,6 +645,7 @@ __device__ __forceinline__ void dn_dx_all(const DevState& s, int c, const double
 // USF: the stress update with the velocities of compute_velocity
 template <int DIM, bool BOX>
 __global__ void __launch_bounds__(128) k_stress(DevState s, double dt) {
+  after_previous();
   constexpr int NV = Elem<DIM>::NV;
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= s.np) return;
@@ -598,6 +666,7 @@ __global__ void __launch_bounds__(128) k_stress(DevState s, double dt) {
 template <int DIM, bool STRESS, int VU, bool BOX>
 __global__ void __launch_bounds__(128, MPM_G2P_MIN_BLOCKS) k_g2p(DevState s, double dt,
                                                                  double beta) {
+  after_previous();
   constexpr int NV = Elem<DIM>::NV;
   constexpr bool FLIP = VU == 0, ASFLIP = VU == 2, TPIC = VU == 3;  // 1 PIC, 4 APIC
   constexpr bool ACC = FLIP || ASFLIP;  // nodal acceleration interpolated
@@ -737,20 +806,7 @@ __global__ void __launch_bounds__(128, MPM_G2P_MIN_BLOCKS) k_g2p(DevState s, dou
     dn_dx_all<DIM, BOX>(s, c, xi, X, D);
     stress_update<DIM>(s, GlobalRow{s, p}, c, nid, D, dt);
   }
-  bool finite = true;
-#pragma unroll
-  for (int d = 0; d < DIM; ++d) finite = finite && isfinite(xn[d]);
-  if (!finite) {
-    raise_err(s, ERR_NONFINITE);
-    s.lost[atomicAdd(s.nlost, 1u)] = (int32_t)p;
-    return;
-  }
-  const int nc = locate_near<DIM, BOX>(s, xn, c);
-  if (nc >= 0) {
-    if (nc != c) s.cell[p] = nc;
-  } else {
-    s.lost[atomicAdd(s.nlost, 1u)] = (int32_t)p;
-  }
+  settle_particle<DIM, BOX>(s, p, xn, c);
 }
 
 // USL G2P + stress update + locate with the block's particle slices staged in
@@ -793,6 +849,7 @@ __global__ void __launch_bounds__(STAGE_T, MPM_G2P_MIN_BLOCKS)
     bulk::mbar_init(&bar[1], 1);
     bulk::fence_barrier_init();
   }
+  after_previous();
   __syncthreads();
   if (t == 0) {
     bulk::mbar_arrive_expect_tx(&bar[0], ROWS_A * T * 8 + T * (4 + 2 + 2));
@@ -891,22 +948,7 @@ __global__ void __launch_bounds__(STAGE_T, MPM_G2P_MIN_BLOCKS)
           bulk::store(s.sv + k * np + p0, svr + k * T, T * 8);
     bulk::store_commit();
   }
-  if (active) {
-    bool finite = true;
-#pragma unroll
-    for (int d = 0; d < DIM; ++d) finite = finite && isfinite(xn[d]);
-    if (!finite) {
-      raise_err(s, ERR_NONFINITE);
-      s.lost[atomicAdd(s.nlost, 1u)] = (int32_t)p;
-    } else {
-      const int nc = locate_near<DIM, BOX>(s, xn, c);
-      if (nc >= 0) {
-        if (nc != c) s.cell[p] = nc;
-      } else {
-        s.lost[atomicAdd(s.nlost, 1u)] = (int32_t)p;
-      }
-    }
-  }
+  if (active) settle_particle<DIM, BOX>(s, p, xn, c);
   if (t == 0) bulk::store_wait_read();
 }
 
@@ -917,6 +959,7 @@ __global__ void __launch_bounds__(STAGE_T, MPM_G2P_MIN_BLOCKS)
 template <int DIM, bool FLIP, bool BOX>
 __global__ void __launch_bounds__(128, MPM_G2P_MIN_BLOCKS) k_g2p_musl(DevState s, double dt,
                                                                       double beta) {
+  after_previous();
   constexpr int NV = Elem<DIM>::NV;
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= s.np) return;
@@ -973,30 +1016,19 @@ __global__ void __launch_bounds__(128, MPM_G2P_MIN_BLOCKS) k_g2p_musl(DevState s
 // MUSL end of step: the new positions replace the old, then locate
 template <int DIM, bool BOX>
 __global__ void __launch_bounds__(128) k_commit_locate(DevState s) {
+  after_previous();
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= s.np) return;
   const int c = s.cell[p];
   if (c < 0) return;
   const int64_t np = s.np;
   double xn[DIM];
-  bool finite = true;
 #pragma unroll
   for (int d = 0; d < DIM; ++d) {
     xn[d] = s.xnext[(int64_t)d * np + p];
     s.pf[(int64_t)(PF<DIM>::X + d) * np + p] = xn[d];
-    finite = finite && isfinite(xn[d]);
   }
-  if (!finite) {
-    raise_err(s, ERR_NONFINITE);
-    s.lost[atomicAdd(s.nlost, 1u)] = (int32_t)p;
-    return;
-  }
-  const int nc = locate_near<DIM, BOX>(s, xn, c);
-  if (nc >= 0) {
-    if (nc != c) s.cell[p] = nc;
-  } else {
-    s.lost[atomicAdd(s.nlost, 1u)] = (int32_t)p;
-  }
+  settle_particle<DIM, BOX>(s, p, xn, c);
 }
 
 // The MohrCoulomb returns deferred by stress_update, one thread per listed
@@ -1007,6 +1039,7 @@ __global__ void __launch_bounds__(128) k_commit_locate(DevState s) {
 // step's grouping.
 template <int DIM>
 __global__ void __launch_bounds__(128, MPM_MC_RETURN_MIN_BLOCKS) k_mc_return(DevState s) {
+  after_previous();
   const unsigned nl = *s.nplastic, n = nl + *s.nplastic_heavy;
   const int64_t np = s.np;
   for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
@@ -1035,21 +1068,26 @@ __global__ void __launch_bounds__(128, MPM_MC_RETURN_MIN_BLOCKS) k_mc_return(Dev
 // contains the point).  Grid-stride over the lost list; usually empty.
 template <int DIM>
 __global__ void k_locate_fallback(DevState s, int remove_lost) {
+  after_previous();
   locate_lost<DIM>(s, remove_lost, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
 inline unsigned nblocks(int64_t n, int threads) { return (unsigned)((n + threads - 1) / threads); }
 
-void counting_sort_impl(const DevState& s, cudaStream_t st) {
+// words: also reset the step's list lengths.  One cluster takes the sort of up
+// to SORT_SMALL_NP particles and SORT_SMALL_CELLS cells.
+void counting_sort_impl(const DevState& s, cudaStream_t st, int words) {
   const int64_t nc = s.ncells;
-  cudaMemsetAsync(s.cnt, 0, sizeof(int32_t) * nc, st);
-  k_count<<<nblocks(s.np, 256), 256, 0, st>>>(s);
-  const int64_t nb = (nc + SCAN_BLOCK - 1) / SCAN_BLOCK;
-  k_scan_local<<<(unsigned)nb, 1024, 0, st>>>(s.cnt, s.start, s.bsum, nc);
-  // block totals (nb <= SCAN_BLOCK is checked at set-up) scanned by one block
-  k_scan_local<<<1, 1024, 0, st>>>(s.bsum, s.bsum + nb, nullptr, nb);
-  k_scan_add<<<nblocks(nc, 256), 256, 0, st>>>(s.start, s.bsum + nb, s.bsum, nc, nb);
-  k_fill<<<nblocks(s.np, 256), 256, 0, st>>>(s);
+  if (s.np <= SORT_SMALL_NP && nc <= SORT_SMALL_CELLS) {
+    launch_dependent(k_sort_small, SORT_CLUSTER, 1024, 0, st, s, words);
+    return;
+  }
+  launch_dependent(k_sort_reset, (unsigned)std::min<int64_t>(nblocks(nc, 1024), 148 * 8), 256, 0, st, s, words);
+  launch_dependent(k_count, nblocks(s.np, 256), 256, 0, st, s);
+  const unsigned nb = nblocks(nc, SCAN_BLOCK);
+  launch_dependent(k_scan_local, nb, 1024, 0, st, s);
+  launch_dependent(k_scan_add, nb, 1024, 0, st, s);
+  launch_dependent(k_fill, nblocks(s.np, 256), 256, 0, st, s);
 }
 
 // Ask for the shared-memory carveout that lets MIN_BLOCKS staged blocks share
@@ -1070,14 +1108,16 @@ template <int DIM, bool BOX>
 void step_impl(const DevState& s, const StepArgs& a, cudaStream_t st, Profiler& pr) {
   const int64_t np = s.np, nn = s.nn;
   if (np == 0) return;
-  cudaMemsetAsync(s.nlost, 0, sizeof(unsigned), st);
-  if (s.sv) cudaMemsetAsync(s.nplastic, 0, 2 * sizeof(unsigned), st);  // and nplastic_heavy
   const unsigned nt = (unsigned)node_block(a);
   const unsigned pb128 = nblocks(np, 128), nb = nblocks(nn, nt);
   const unsigned mcb = (unsigned)std::min<int64_t>(nblocks(np, 128), 148 * return_blocks(a));
   auto mc_returns = [&]() {
     if (!s.sv) return;
     pr.begin(K_MC_RETURN, st);
+    // A plain launch: the return keeps part of its state in local memory and needs
+    // the L1 that the staged G2P gave to shared memory.  Blocks that an SM takes
+    // on while G2P's last ones run keep that split to their end: a flowing 0.8M-
+    // particle step took 323 us with a dependent launch here, 263 with this one.
     k_mc_return<DIM><<<mcb, 128, 0, st>>>(s);
     pr.end(K_MC_RETURN, st);
   };
@@ -1087,11 +1127,9 @@ void step_impl(const DevState& s, const StepArgs& a, cudaStream_t st, Profiler& 
       constexpr int AFF = decltype(aff)::value;
       constexpr int TT = p2g_tile_t<BOX, AFF>();
       if (BOX && !AFF && tile_threads(a, BOX) == 128)
-        k_p2g_tiles<DIM, MODE, BOX, AFF, 128><<<nblocks(s.ncells, 128 / Elem<DIM>::NV), 128, 0, st>>>(
-            s, a.g[0], a.g[1], a.g[2]);
+        launch_dependent(k_p2g_tiles<DIM, MODE, BOX, AFF, 128>, nblocks(s.ncells, 128 / Elem<DIM>::NV), 128, 0, st, s, a.g[0], a.g[1], a.g[2]);
       else
-        k_p2g_tiles<DIM, MODE, BOX, AFF><<<nblocks(s.ncells, TT / Elem<DIM>::NV), TT, 0, st>>>(
-            s, a.g[0], a.g[1], a.g[2]);
+        launch_dependent(k_p2g_tiles<DIM, MODE, BOX, AFF>, nblocks(s.ncells, TT / Elem<DIM>::NV), TT, 0, st, s, a.g[0], a.g[1], a.g[2]);
     };
     if constexpr (MODE != 1) {  // the mass-momentum mapping velocity
       if (a.vupd == 2 || a.vupd == 4) return launch(std::integral_constant<int, 1>{});
@@ -1104,29 +1142,29 @@ void step_impl(const DevState& s, const StepArgs& a, cudaStream_t st, Profiler& 
   auto g2p = [&](auto stress) {
     constexpr bool STRESS = decltype(stress)::value;
     switch (a.vupd) {
-      case 0: k_g2p<DIM, STRESS, 0, BOX><<<pb128, 128, 0, st>>>(s, a.dt, a.beta); break;
-      case 1: k_g2p<DIM, STRESS, 1, BOX><<<pb128, 128, 0, st>>>(s, a.dt, a.beta); break;
-      case 2: k_g2p<DIM, STRESS, 2, BOX><<<pb128, 128, 0, st>>>(s, a.dt, a.beta); break;
-      case 3: k_g2p<DIM, STRESS, 3, BOX><<<pb128, 128, 0, st>>>(s, a.dt, a.beta); break;
-      default: k_g2p<DIM, STRESS, 4, BOX><<<pb128, 128, 0, st>>>(s, a.dt, a.beta); break;
+      case 0: launch_dependent(k_g2p<DIM, STRESS, 0, BOX>, pb128, 128, 0, st, s, a.dt, a.beta); break;
+      case 1: launch_dependent(k_g2p<DIM, STRESS, 1, BOX>, pb128, 128, 0, st, s, a.dt, a.beta); break;
+      case 2: launch_dependent(k_g2p<DIM, STRESS, 2, BOX>, pb128, 128, 0, st, s, a.dt, a.beta); break;
+      case 3: launch_dependent(k_g2p<DIM, STRESS, 3, BOX>, pb128, 128, 0, st, s, a.dt, a.beta); break;
+      default: launch_dependent(k_g2p<DIM, STRESS, 4, BOX>, pb128, 128, 0, st, s, a.dt, a.beta); break;
     }
   };
   if (a.scheme == 1 && a.phase == 2) goto usl_second_half;
-  pr.begin(K_SORT, st, SORT_KERNELS);
-  counting_sort_impl(s, st);
+  pr.begin(K_SORT, st, sort_kernels(s));
+  counting_sort_impl(s, st, 1);
   pr.end(K_SORT, st);
   if (a.scheme == 2) {  // MUSL (mpm_scheme_musl.tcc)
     pr.begin(K_P2G, st);
     p2g(std::integral_constant<int, 2>{});
     pr.end(K_P2G, st);
     pr.begin(K_NODES_VEL, st);
-    k_nodes<DIM, 1><<<nb, nt, 0, st>>>(s, a.dt, a.damping);
+    launch_dependent(k_nodes<DIM, 1>, nb, nt, 0, st, s, a.dt, a.damping);
     pr.end(K_NODES_VEL, st);
     pr.begin(K_G2P, st);
     if (a.flip)
-      k_g2p_musl<DIM, true, BOX><<<pb128, 128, 0, st>>>(s, a.dt, a.beta);
+      launch_dependent(k_g2p_musl<DIM, true, BOX>, pb128, 128, 0, st, s, a.dt, a.beta);
     else
-      k_g2p_musl<DIM, false, BOX><<<pb128, 128, 0, st>>>(s, a.dt, a.beta);
+      launch_dependent(k_g2p_musl<DIM, false, BOX>, pb128, 128, 0, st, s, a.dt, a.beta);
     pr.end(K_G2P, st);
     // mass and momentum again with the updated velocities, nodal velocity,
     // then the stress update (mpm_scheme_musl.tcc:13-35)
@@ -1134,14 +1172,14 @@ void step_impl(const DevState& s, const StepArgs& a, cudaStream_t st, Profiler& 
     p2g(std::integral_constant<int, 0>{});
     pr.end(K_P2G_FORCES, st);
     pr.begin(K_NODES_ACC, st);
-    k_nodes<DIM, 0><<<nb, nt, 0, st>>>(s, a.dt, a.damping);
+    launch_dependent(k_nodes<DIM, 0>, nb, nt, 0, st, s, a.dt, a.damping);
     pr.end(K_NODES_ACC, st);
     pr.begin(K_STRESS, st);
-    k_stress<DIM, BOX><<<pb128, 128, 0, st>>>(s, a.dt);
+    launch_dependent(k_stress<DIM, BOX>, pb128, 128, 0, st, s, a.dt);
     pr.end(K_STRESS, st);
     mc_returns();
     pr.begin(K_LOCATE, st);
-    k_commit_locate<DIM, BOX><<<pb128, 128, 0, st>>>(s);
+    launch_dependent(k_commit_locate<DIM, BOX>, pb128, 128, 0, st, s);
     pr.end(K_LOCATE, st);
   } else if (a.scheme == 1) {  // USL
     pr.begin(K_P2G, st);
@@ -1150,7 +1188,7 @@ void step_impl(const DevState& s, const StepArgs& a, cudaStream_t st, Profiler& 
     if (a.phase == 1) return;
   usl_second_half:
     pr.begin(K_NODES_VEL, st);
-    k_nodes<DIM, 1><<<nb, nt, 0, st>>>(s, a.dt, a.damping);
+    launch_dependent(k_nodes<DIM, 1>, nb, nt, 0, st, s, a.dt, a.damping);
     pr.end(K_NODES_VEL, st);
     pr.begin(K_G2P, st);
     const size_t sm = staged_smem_bytes<DIM>(s.sv != nullptr);
@@ -1158,10 +1196,10 @@ void step_impl(const DevState& s, const StepArgs& a, cudaStream_t st, Profiler& 
       g2p(std::true_type{});
     } else if (a.flip) {
       prefer_shared_memory<k_g2p_staged<DIM, true, BOX>>();
-      k_g2p_staged<DIM, true, BOX><<<pb128, STAGE_T, sm, st>>>(s, a.dt, a.beta);
+      launch_dependent(k_g2p_staged<DIM, true, BOX>, pb128, STAGE_T, sm, st, s, a.dt, a.beta);
     } else {
       prefer_shared_memory<k_g2p_staged<DIM, false, BOX>>();
-      k_g2p_staged<DIM, false, BOX><<<pb128, STAGE_T, sm, st>>>(s, a.dt, a.beta);
+      launch_dependent(k_g2p_staged<DIM, false, BOX>, pb128, STAGE_T, sm, st, s, a.dt, a.beta);
     }
     pr.end(K_G2P, st);
     mc_returns();
@@ -1170,25 +1208,27 @@ void step_impl(const DevState& s, const StepArgs& a, cudaStream_t st, Profiler& 
     p2g(std::integral_constant<int, 0>{});
     pr.end(K_P2G, st);
     pr.begin(K_NODES_VEL, st);
-    k_nodes<DIM, 0><<<nb, nt, 0, st>>>(s, a.dt, a.damping);
+    launch_dependent(k_nodes<DIM, 0>, nb, nt, 0, st, s, a.dt, a.damping);
     pr.end(K_NODES_VEL, st);
     pr.begin(K_STRESS, st);
-    k_stress<DIM, BOX><<<pb128, 128, 0, st>>>(s, a.dt);
+    launch_dependent(k_stress<DIM, BOX>, pb128, 128, 0, st, s, a.dt);
     pr.end(K_STRESS, st);
     mc_returns();
     pr.begin(K_P2G_FORCES, st);
     p2g(std::integral_constant<int, 1>{});
     pr.end(K_P2G_FORCES, st);
     pr.begin(K_NODES_ACC, st);
-    k_nodes<DIM, 2><<<nb, nt, 0, st>>>(s, a.dt, a.damping);
+    launch_dependent(k_nodes<DIM, 2>, nb, nt, 0, st, s, a.dt, a.damping);
     pr.end(K_NODES_ACC, st);
     pr.begin(K_G2P, st);
     g2p(std::false_type{});
     pr.end(K_G2P, st);
   }
-  pr.begin(K_LOCATE, st);
-  k_locate_fallback<DIM><<<148, 128, 0, st>>>(s, a.remove_lost);
-  pr.end(K_LOCATE, st);
+  if (!BOX) {  // on a grid every particle settled itself
+    pr.begin(K_LOCATE, st);
+    launch_dependent(k_locate_fallback<DIM>, 148, 128, 0, st, s, a.remove_lost);
+    pr.end(K_LOCATE, st);
+  }
 }
 
 template <int DIM>
@@ -1225,7 +1265,7 @@ void launch_step_fp64(int dim, const DevState& s, const StepArgs& a, cudaStream_
     s.structured ? step_impl<3, true>(s, a, st, prof) : step_impl<3, false>(s, a, st, prof);
 }
 
-void counting_sort(const DevState& s, cudaStream_t st) { counting_sort_impl(s, st); }
+void counting_sort(const DevState& s, cudaStream_t st, int words) { counting_sort_impl(s, st, words); }
 
 // The first half of a USL step: sort, P2G of mass, momentum and forces, and the
 // node update (FLIP / PIC mapping velocity), leaving the cell-slot partials and
@@ -1233,14 +1273,13 @@ void counting_sort(const DevState& s, cudaStream_t st) { counting_sort_impl(s, s
 // adjoint recomputes these from a stored step-start state.
 void launch_p2g_nodes_fp64(int dim, const DevState& s, const StepArgs& a, cudaStream_t st) {
   if (s.np == 0) return;
-  counting_sort_impl(s, st);
+  counting_sort_impl(s, st, 0);
   auto run = [&](auto dimc, auto boxc) {
     constexpr int DIM = decltype(dimc)::value;
     constexpr bool BOX = decltype(boxc)::value;
     constexpr int TT = p2g_tile_t<BOX, 0>();
-    k_p2g_tiles<DIM, 2, BOX, 0><<<nblocks(s.ncells, TT / Elem<DIM>::NV), TT, 0, st>>>(
-        s, a.g[0], a.g[1], a.g[2]);
-    k_nodes<DIM, 1><<<nblocks(s.nn, 256), 256, 0, st>>>(s, a.dt, a.damping);
+    launch_dependent(k_p2g_tiles<DIM, 2, BOX, 0>, nblocks(s.ncells, TT / Elem<DIM>::NV), TT, 0, st, s, a.g[0], a.g[1], a.g[2]);
+    launch_dependent(k_nodes<DIM, 1>, nblocks(s.nn, 256), 256, 0, st, s, a.dt, a.damping);
   };
   if (dim == 2)
     s.structured ? run(std::integral_constant<int, 2>{}, std::true_type{})
@@ -1252,9 +1291,9 @@ void launch_p2g_nodes_fp64(int dim, const DevState& s, const StepArgs& a, cudaSt
 
 void launch_locate_fallback(int dim, const DevState& s, int remove_lost, cudaStream_t st) {
   if (dim == 2)
-    k_locate_fallback<2><<<148, 128, 0, st>>>(s, remove_lost);
+    launch_dependent(k_locate_fallback<2>, 148, 128, 0, st, s, remove_lost);
   else
-    k_locate_fallback<3><<<148, 128, 0, st>>>(s, remove_lost);
+    launch_dependent(k_locate_fallback<3>, 148, 128, 0, st, s, remove_lost);
 }
 
 void launch_material_batch_fp64(int dim, int64_t n, const MaterialParams& m, const double* stress,

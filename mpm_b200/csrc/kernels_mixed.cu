@@ -28,6 +28,7 @@
 #include "mpm_device.cuh"
 #include "mpm_grid.cuh"
 #include "mpm_kernels.h"
+#include "mpm_launch.cuh"
 #include "mpm_return.cuh"
 #include "mpm_state.cuh"
 
@@ -419,6 +420,7 @@ __device__ __forceinline__ void p2g_tile_mixed(const DevState& s, int64_t bx) {
 template <int DIM, int MODE, bool BOX, int T = p2g_tile_t<BOX>(), int AFF = 0>
 __global__ void __launch_bounds__(T, (mixed_tile_min_blocks<BOX, T, AFF>()))
     k_p2g_tiles_mixed(DevState s) {
+  after_previous();
   p2g_tile_mixed<DIM, MODE, BOX, T, AFF>(s, blockIdx.x);
 }
 
@@ -547,6 +549,7 @@ __device__ __forceinline__ void node_update_mixed(const DevState& s, double dt, 
 template <int DIM, int MODE>
 __global__ void __launch_bounds__(256, MPM_MIXED_NODES_MIN_BLOCKS) k_nodes_mixed(DevState s, double dt, double damping, double g0,
                                                         double g1, double g2) {
+  after_previous();
   const double g[3] = {g0, g1, g2};
   node_update_mixed<DIM, MODE>(s, dt, damping, g, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
 }
@@ -901,6 +904,7 @@ __device__ __forceinline__ void gather_particle(const DevState& s, int c, const 
 
 template <int DIM, bool BOX>
 __global__ void __launch_bounds__(128) k_stress_mixed(DevState s, float dt) {
+  after_previous();
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= s.np) return;
   const int c = s.cell[p];
@@ -920,6 +924,7 @@ __global__ void __launch_bounds__(128) k_stress_mixed(DevState s, float dt) {
 template <int DIM, bool STRESS, bool FLIP, bool BOX, bool MUSL = false>
 __global__ void __launch_bounds__(128, MPM_MIXED_G2P_MIN_BLOCKS)
     k_g2p_mixed(DevState s, double dt, float beta) {
+  after_previous();
   static_assert(!(MUSL && STRESS), "MUSL updates the stress after its second mapping");
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= s.np) return;
@@ -966,20 +971,7 @@ __global__ void __launch_bounds__(128, MPM_MIXED_G2P_MIN_BLOCKS)
   for (int d = 0; d < DIM; ++d) set_pmf<DIM>(s, PM<DIM>::V + d, p, v[d]);
   if constexpr (MUSL) return;
   if constexpr (STRESS) stress_update_mixed<DIM>(s, MGlobalRow<DIM>{s, p}, grad, dtf);
-  bool finite = true;
-#pragma unroll
-  for (int d = 0; d < DIM; ++d) finite = finite && isfinite(xn[d]);
-  if (!finite) {
-    raise_err(s, ERR_NONFINITE);
-    s.lost[atomicAdd(s.nlost, 1u)] = (int32_t)p;
-    return;
-  }
-  const int nc = locate_near<DIM, BOX>(s, xn, c);
-  if (nc >= 0) {
-    if (nc != c) s.cell[p] = nc;
-  } else {
-    s.lost[atomicAdd(s.nlost, 1u)] = (int32_t)p;
-  }
+  settle_particle<DIM, BOX>(s, p, xn, c);
 }
 
 // G2P of the velocity updates that carry a mapping matrix (particle.tcc:
@@ -992,6 +984,7 @@ __global__ void __launch_bounds__(128, MPM_MIXED_G2P_MIN_BLOCKS)
 template <int DIM, bool STRESS, int VU, bool BOX>
 __global__ void __launch_bounds__(128, MPM_MIXED_AFFINE_G2P_MIN_BLOCKS)
     k_g2p_mixed_affine(DevState s, double dt, float beta) {
+  after_previous();
   static_assert(VU >= 2, "the mapping-matrix updates");
   constexpr int NV = Elem<DIM>::NV;
   constexpr bool ASFLIP = VU == 2, TPIC = VU == 3;  // 4 APIC
@@ -1124,49 +1117,25 @@ __global__ void __launch_bounds__(128, MPM_MIXED_AFFINE_G2P_MIN_BLOCKS)
   for (int d = 0; d < DIM; ++d) set_pmf<DIM>(s, PM<DIM>::V + d, p, v[d]);
   if constexpr (STRESS)
     stress_update_mixed<DIM>(s, MGlobalRow<DIM>{s, p}, velocity_gradient<DIM>(s, c, nid, D), dtf);
-  bool finite = true;
-#pragma unroll
-  for (int d = 0; d < DIM; ++d) finite = finite && isfinite(xn[d]);
-  if (!finite) {
-    raise_err(s, ERR_NONFINITE);
-    s.lost[atomicAdd(s.nlost, 1u)] = (int32_t)p;
-    return;
-  }
-  const int nc = locate_near<DIM, BOX>(s, xn, c);
-  if (nc >= 0) {
-    if (nc != c) s.cell[p] = nc;
-  } else {
-    s.lost[atomicAdd(s.nlost, 1u)] = (int32_t)p;
-  }
+  settle_particle<DIM, BOX>(s, p, xn, c);
 }
 
 // MUSL end of step: the new positions (FP64) replace the old, then locate
 template <int DIM, bool BOX>
 __global__ void __launch_bounds__(128) k_commit_locate_mixed(DevState s) {
+  after_previous();
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= s.np) return;
   const int c = s.cell[p];
   if (c < 0) return;
   const int64_t np = s.np;
   double xn[DIM];
-  bool finite = true;
 #pragma unroll
   for (int d = 0; d < DIM; ++d) {
     xn[d] = s.xnext[(int64_t)d * np + p];
     s.pf[(int64_t)(PDX<DIM>::X + d) * np + p] = xn[d];
-    finite = finite && isfinite(xn[d]);
   }
-  if (!finite) {
-    raise_err(s, ERR_NONFINITE);
-    s.lost[atomicAdd(s.nlost, 1u)] = (int32_t)p;
-    return;
-  }
-  const int nc = locate_near<DIM, BOX>(s, xn, c);
-  if (nc >= 0) {
-    if (nc != c) s.cell[p] = nc;
-  } else {
-    s.lost[atomicAdd(s.nlost, 1u)] = (int32_t)p;
-  }
+  settle_particle<DIM, BOX>(s, p, xn, c);
 }
 
 // USL G2P + stress update + locate with the block's particle slices staged in
@@ -1289,22 +1258,7 @@ __device__ __forceinline__ void g2p_staged_block_mixed(const DevState& s, double
           bulk::store(s.svf + k * np + p0, svr + k * T, T * 4);
     bulk::store_commit();
   }
-  if (active) {
-    bool finite = true;
-#pragma unroll
-    for (int d = 0; d < DIM; ++d) finite = finite && isfinite(xn[d]);
-    if (!finite) {
-      raise_err(s, ERR_NONFINITE);
-      s.lost[atomicAdd(s.nlost, 1u)] = (int32_t)p;
-    } else {
-      const int nc = locate_near<DIM, BOX>(s, xn, c);
-      if (nc >= 0) {
-        if (nc != c) s.cell[p] = nc;
-      } else {
-        s.lost[atomicAdd(s.nlost, 1u)] = (int32_t)p;
-      }
-    }
-  }
+  if (active) settle_particle<DIM, BOX>(s, p, xn, c);
   if (t == 0) {
     if constexpr (WRITES_DONE)
       bulk::store_wait_all();
@@ -1324,6 +1278,7 @@ __global__ void __launch_bounds__(MSTAGE_T, MPM_MIXED_G2P_MIN_BLOCKS)
     bulk::mbar_init(&bar[1], 1);
     bulk::fence_barrier_init();
   }
+  after_previous();
   g2p_staged_block_mixed<DIM, FLIP, BOX>(s, dt, beta, blockIdx.x, smem, bar, 0u, timed_out);
 }
 
@@ -1391,6 +1346,7 @@ __device__ __forceinline__ void mc_return_mixed_range(const DevState& s, unsigne
 
 template <int DIM>
 __global__ void __launch_bounds__(128, MPM_MC_RETURN_MIN_BLOCKS) k_mc_return_mixed(DevState s) {
+  after_previous();
   mc_return_mixed_range<DIM>(s, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
@@ -1453,7 +1409,7 @@ __device__ __forceinline__ int32_t block_total(const int32_t* bsum, int64_t coun
 // (the P2G tiles have 128 threads; each cell's particle ids are sorted before
 // they are added, so the slot order the counting sort leaves does not matter):
 //   count | scan chunks | chunk prefixes | fill | P2G | nodes |
-//   G2P + stress (and the next step's counts zeroed) | returns [| locate]
+//   G2P + stress (and the next step's counts zeroed) | returns
 template <int DIM, bool FLIP>
 __global__ void __launch_bounds__(MSTAGE_T, DIM == 2 ? MPM_PERSISTENT_MIN_BLOCKS_2D : MPM_PERSISTENT_MIN_BLOCKS_3D)
     k_steps_persistent_mixed(DevState s, StepArgs a, PersistentArgs q) {
@@ -1487,7 +1443,6 @@ __global__ void __launch_bounds__(MSTAGE_T, DIM == 2 ? MPM_PERSISTENT_MIN_BLOCKS
     const double g[3] = {gm * q.gravity[0], gm * q.gravity[1], gm * q.gravity[2]};
     // counting sort
     if (blockIdx.x == 0 && t == 0) {
-      *s.nlost = 0;
       if (s.svf) *s.nplastic = *s.nplastic_heavy = 0;
     }
     for (int64_t b = blockIdx.x; b < pblocks; b += G) count_particle(s, b * T + t);
@@ -1523,10 +1478,6 @@ __global__ void __launch_bounds__(MSTAGE_T, DIM == 2 ? MPM_PERSISTENT_MIN_BLOCKS
       mc_return_mixed_range<DIM>(s, gi, gs);
       if (!grid_barrier(s, q.barrier, G, gen, go)) return;
     }
-    if (ld_acquire_gpu(s.nlost) != 0) {  // the same value in every block
-      locate_lost<DIM>(s, a.remove_lost, gi, gs);
-      if (!grid_barrier(s, q.barrier, G, gen, go)) return;
-    }
   }
   if (blockIdx.x == 0 && t == 0) *q.step = step0 + q.nsteps;
 }
@@ -1557,8 +1508,6 @@ template <int DIM, bool BOX>
 void step_mixed(const DevState& s, const StepArgs& a, cudaStream_t st, Profiler& pr) {
   const int64_t np = s.np, nn = s.nn;
   if (np == 0) return;
-  cudaMemsetAsync(s.nlost, 0, sizeof(unsigned), st);
-  if (s.svf) cudaMemsetAsync(s.nplastic, 0, 2 * sizeof(unsigned), st);  // and nplastic_heavy
   const unsigned nt = (unsigned)node_block(a);
   const unsigned pb = nblk(np, 128), nb = nblk(nn, nt);
   const unsigned mcap = 148u * (unsigned)return_blocks(a);
@@ -1569,53 +1518,57 @@ void step_mixed(const DevState& s, const StepArgs& a, cudaStream_t st, Profiler&
     constexpr int NV = Elem<DIM>::NV;
     if constexpr (MODE != 1) {  // the mass-momentum mapping velocity (128-thread tiles)
       if (a.vupd == 2 || a.vupd == 4) {
-        k_p2g_tiles_mixed<DIM, MODE, BOX, 128, 1><<<nblk(s.ncells, 128 / NV), 128, 0, st>>>(s);
+        launch_dependent(k_p2g_tiles_mixed<DIM, MODE, BOX, 128, 1>, nblk(s.ncells, 128 / NV), 128, 0, st, s);
         return;
       }
       if (a.vupd == 3) {
-        k_p2g_tiles_mixed<DIM, MODE, BOX, 128, 2><<<nblk(s.ncells, 128 / NV), 128, 0, st>>>(s);
+        launch_dependent(k_p2g_tiles_mixed<DIM, MODE, BOX, 128, 2>, nblk(s.ncells, 128 / NV), 128, 0, st, s);
         return;
       }
     }
     if (BOX && tile_threads(a, BOX) == 128)
-      k_p2g_tiles_mixed<DIM, MODE, BOX, 128><<<nblk(s.ncells, 128 / NV), 128, 0, st>>>(s);
+      launch_dependent(k_p2g_tiles_mixed<DIM, MODE, BOX, 128>, nblk(s.ncells, 128 / NV), 128, 0, st, s);
     else
-      k_p2g_tiles_mixed<DIM, MODE, BOX><<<nblk(s.ncells, p2g_tile_t<BOX>() / NV), p2g_tile_t<BOX>(),
-                                          0, st>>>(s);
+      launch_dependent(k_p2g_tiles_mixed<DIM, MODE, BOX>, nblk(s.ncells, p2g_tile_t<BOX>() / NV),
+                       p2g_tile_t<BOX>(), 0, st, s);
   };
   // G2P of the mapping-matrix updates (ASFLIP 2, TPIC 3, APIC 4)
   auto g2p_affine = [&](auto stress) {
     constexpr bool STRESS = decltype(stress)::value;
     const float b = (float)a.beta;
     if (a.vupd == 2)
-      k_g2p_mixed_affine<DIM, STRESS, 2, BOX><<<pb, 128, 0, st>>>(s, a.dt, b);
+      launch_dependent(k_g2p_mixed_affine<DIM, STRESS, 2, BOX>, pb, 128, 0, st, s, a.dt, b);
     else if (a.vupd == 3)
-      k_g2p_mixed_affine<DIM, STRESS, 3, BOX><<<pb, 128, 0, st>>>(s, a.dt, b);
+      launch_dependent(k_g2p_mixed_affine<DIM, STRESS, 3, BOX>, pb, 128, 0, st, s, a.dt, b);
     else
-      k_g2p_mixed_affine<DIM, STRESS, 4, BOX><<<pb, 128, 0, st>>>(s, a.dt, b);
+      launch_dependent(k_g2p_mixed_affine<DIM, STRESS, 4, BOX>, pb, 128, 0, st, s, a.dt, b);
   };
   auto mc_returns = [&]() {
     if (!s.svf) return;
     pr.begin(K_MC_RETURN, st);
+    // A plain launch: the return keeps part of its state in local memory and needs
+    // the L1 that the staged G2P gave to shared memory.  Blocks that an SM takes
+    // on while G2P's last ones run keep that split to their end: a flowing 0.8M-
+    // particle step took 323 us with a dependent launch here, 263 with this one.
     k_mc_return_mixed<DIM><<<mcb, 128, 0, st>>>(s);
     pr.end(K_MC_RETURN, st);
   };
   if (a.scheme == 1 && a.phase == 2) goto usl_second_half;
-  pr.begin(K_SORT, st, SORT_KERNELS);
-  counting_sort(s, st);
+  pr.begin(K_SORT, st, sort_kernels(s));
+  counting_sort(s, st, 1);
   pr.end(K_SORT, st);
   if (a.scheme == 2) {  // MUSL (mpm_scheme_musl.tcc:20-35)
     pr.begin(K_P2G, st);
     p2g(std::integral_constant<int, 2>{});
     pr.end(K_P2G, st);
     pr.begin(K_NODES_VEL, st);
-    k_nodes_mixed<DIM, 1><<<nb, nt, 0, st>>>(s, a.dt, a.damping, a.g[0], a.g[1], a.g[2]);
+    launch_dependent(k_nodes_mixed<DIM, 1>, nb, nt, 0, st, s, a.dt, a.damping, a.g[0], a.g[1], a.g[2]);
     pr.end(K_NODES_VEL, st);
     pr.begin(K_G2P, st);
     if (a.flip)
-      k_g2p_mixed<DIM, false, true, BOX, true><<<pb, 128, 0, st>>>(s, a.dt, (float)a.beta);
+      launch_dependent(k_g2p_mixed<DIM, false, true, BOX, true>, pb, 128, 0, st, s, a.dt, (float)a.beta);
     else
-      k_g2p_mixed<DIM, false, false, BOX, true><<<pb, 128, 0, st>>>(s, a.dt, (float)a.beta);
+      launch_dependent(k_g2p_mixed<DIM, false, false, BOX, true>, pb, 128, 0, st, s, a.dt, (float)a.beta);
     pr.end(K_G2P, st);
     // mass and momentum again with the updated velocities, nodal velocity,
     // then the stress update at the step's positions
@@ -1623,14 +1576,14 @@ void step_mixed(const DevState& s, const StepArgs& a, cudaStream_t st, Profiler&
     p2g(std::integral_constant<int, 0>{});
     pr.end(K_P2G_FORCES, st);
     pr.begin(K_NODES_ACC, st);
-    k_nodes_mixed<DIM, 0><<<nb, nt, 0, st>>>(s, a.dt, a.damping, a.g[0], a.g[1], a.g[2]);
+    launch_dependent(k_nodes_mixed<DIM, 0>, nb, nt, 0, st, s, a.dt, a.damping, a.g[0], a.g[1], a.g[2]);
     pr.end(K_NODES_ACC, st);
     pr.begin(K_STRESS, st);
-    k_stress_mixed<DIM, BOX><<<pb, 128, 0, st>>>(s, (float)a.dt);
+    launch_dependent(k_stress_mixed<DIM, BOX>, pb, 128, 0, st, s, (float)a.dt);
     pr.end(K_STRESS, st);
     mc_returns();
     pr.begin(K_LOCATE, st);
-    k_commit_locate_mixed<DIM, BOX><<<pb, 128, 0, st>>>(s);
+    launch_dependent(k_commit_locate_mixed<DIM, BOX>, pb, 128, 0, st, s);
     pr.end(K_LOCATE, st);
   } else if (a.scheme == 1) {  // USL
     pr.begin(K_P2G, st);
@@ -1639,7 +1592,7 @@ void step_mixed(const DevState& s, const StepArgs& a, cudaStream_t st, Profiler&
     if (a.phase == 1) return;
   usl_second_half:
     pr.begin(K_NODES_VEL, st);
-    k_nodes_mixed<DIM, 1><<<nb, nt, 0, st>>>(s, a.dt, a.damping, a.g[0], a.g[1], a.g[2]);
+    launch_dependent(k_nodes_mixed<DIM, 1>, nb, nt, 0, st, s, a.dt, a.damping, a.g[0], a.g[1], a.g[2]);
     pr.end(K_NODES_VEL, st);
     pr.begin(K_G2P, st);
     const size_t sm = mixed_staged_smem_bytes<DIM>(s.svf != nullptr);
@@ -1647,10 +1600,10 @@ void step_mixed(const DevState& s, const StepArgs& a, cudaStream_t st, Profiler&
       g2p_affine(std::true_type{});
     } else if (a.flip) {
       prefer_shared_memory<k_g2p_mixed_staged<DIM, true, BOX>>();
-      k_g2p_mixed_staged<DIM, true, BOX><<<pb, MSTAGE_T, sm, st>>>(s, a.dt, (float)a.beta);
+      launch_dependent(k_g2p_mixed_staged<DIM, true, BOX>, pb, MSTAGE_T, sm, st, s, a.dt, (float)a.beta);
     } else {
       prefer_shared_memory<k_g2p_mixed_staged<DIM, false, BOX>>();
-      k_g2p_mixed_staged<DIM, false, BOX><<<pb, MSTAGE_T, sm, st>>>(s, a.dt, (float)a.beta);
+      launch_dependent(k_g2p_mixed_staged<DIM, false, BOX>, pb, MSTAGE_T, sm, st, s, a.dt, (float)a.beta);
     }
     pr.end(K_G2P, st);
     mc_returns();
@@ -1659,30 +1612,32 @@ void step_mixed(const DevState& s, const StepArgs& a, cudaStream_t st, Profiler&
     p2g(std::integral_constant<int, 0>{});
     pr.end(K_P2G, st);
     pr.begin(K_NODES_VEL, st);
-    k_nodes_mixed<DIM, 0><<<nb, nt, 0, st>>>(s, a.dt, a.damping, a.g[0], a.g[1], a.g[2]);
+    launch_dependent(k_nodes_mixed<DIM, 0>, nb, nt, 0, st, s, a.dt, a.damping, a.g[0], a.g[1], a.g[2]);
     pr.end(K_NODES_VEL, st);
     pr.begin(K_STRESS, st);
-    k_stress_mixed<DIM, BOX><<<pb, 128, 0, st>>>(s, (float)a.dt);
+    launch_dependent(k_stress_mixed<DIM, BOX>, pb, 128, 0, st, s, (float)a.dt);
     pr.end(K_STRESS, st);
     mc_returns();
     pr.begin(K_P2G_FORCES, st);
     p2g(std::integral_constant<int, 1>{});
     pr.end(K_P2G_FORCES, st);
     pr.begin(K_NODES_ACC, st);
-    k_nodes_mixed<DIM, 2><<<nb, nt, 0, st>>>(s, a.dt, a.damping, a.g[0], a.g[1], a.g[2]);
+    launch_dependent(k_nodes_mixed<DIM, 2>, nb, nt, 0, st, s, a.dt, a.damping, a.g[0], a.g[1], a.g[2]);
     pr.end(K_NODES_ACC, st);
     pr.begin(K_G2P, st);
     if (a.vupd >= 2)
       g2p_affine(std::false_type{});
     else if (a.flip)
-      k_g2p_mixed<DIM, false, true, BOX><<<pb, 128, 0, st>>>(s, a.dt, (float)a.beta);
+      launch_dependent(k_g2p_mixed<DIM, false, true, BOX>, pb, 128, 0, st, s, a.dt, (float)a.beta);
     else
-      k_g2p_mixed<DIM, false, false, BOX><<<pb, 128, 0, st>>>(s, a.dt, (float)a.beta);
+      launch_dependent(k_g2p_mixed<DIM, false, false, BOX>, pb, 128, 0, st, s, a.dt, (float)a.beta);
     pr.end(K_G2P, st);
   }
-  pr.begin(K_LOCATE, st);
-  launch_locate_fallback(DIM, s, a.remove_lost, st);
-  pr.end(K_LOCATE, st);
+  if (!BOX) {  // on a grid every particle settled itself
+    pr.begin(K_LOCATE, st);
+    launch_locate_fallback(DIM, s, a.remove_lost, st);
+    pr.end(K_LOCATE, st);
+  }
 }
 
 }  // namespace

@@ -545,6 +545,25 @@ __device__ __forceinline__ int locate_box(const DevState& s, const double* x, in
   return DIM == 2 ? to[0] + s.gcells[0] * to[1] : to[0] + s.gcells[0] * (to[1] + s.gcells[1] * to[2]);
 }
 
+// The exhaustive search of a tensor-product grid (mesh.tcc:1136-1148 over all
+// cells): the first cell in id order that holds x, or -1.  Only the intervals
+// around x's own can hold it, per axis.
+template <int DIM>
+__device__ __forceinline__ int locate_box_anywhere(const DevState& s, const double* x) {
+  int to[3] = {0, 0, 0};
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) {
+    if (!(x[d] == x[d])) return -1;
+    const int at = axis_interval(s.axis[d], s.gcells[d], x[d]);
+    const int hi = at + 1 < s.gcells[d] ? at + 1 : at;
+    int i = at > 0 ? at - 1 : 0;
+    while (i <= hi && !in_interval(s.axcell[d], i, x[d])) ++i;
+    if (i > hi) return -1;
+    to[d] = i;
+  }
+  return DIM == 2 ? to[0] + s.gcells[0] * to[1] : to[0] + s.gcells[0] * (to[1] + s.gcells[1] * to[2]);
+}
+
 // the search of a general mesh over its neighbour lists
 template <int DIM>
 __device__ __forceinline__ int locate_general(const DevState& s, const double* x, int c) {
@@ -573,6 +592,31 @@ __device__ __forceinline__ int locate_near(const DevState& s, const double* x, i
   }
 }
 
+// The end of particle p's step at its new position xn from cell c: the locate
+// and its errors.  On a tensor-product grid the exhaustive search is a few
+// table reads, so the particle's own thread makes it; on a general mesh the
+// particle is listed for k_locate_fallback.
+template <int DIM, bool BOX>
+__device__ __forceinline__ void settle_particle(const DevState& s, int64_t p, const double* xn, int c) {
+  bool finite = true;
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) finite = finite && isfinite(xn[d]);
+  if (!finite) raise_err(s, ERR_NONFINITE);
+  int nc = finite ? locate_near<DIM, BOX>(s, xn, c) : -1;
+  if (nc < 0) {
+    if constexpr (BOX) {
+      nc = locate_box_anywhere<DIM>(s, xn);
+      if (nc < 0 && !s.remove_lost) {
+        raise_err(s, ERR_OUTSIDE);
+        return;
+      }
+    } else {
+      s.lost[atomicAdd(s.nlost, 1u)] = (int32_t)p;
+      return;
+    }
+  }
+  if (nc != c) s.cell[p] = nc;
+}
 
 // ------------------------------------------------------------ counting sort
 // The passes of the per-step counting sort of particles by cell, as bodies

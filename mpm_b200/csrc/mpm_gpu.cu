@@ -789,7 +789,7 @@ void upload_mesh(mpm_gpu_t h) {
   h->d_cnt.alloc(h->ncells);
   h->d_start.alloc(h->ncells + 1);
   const int64_t nb = (h->ncells + SCAN_BLOCK - 1) / SCAN_BLOCK;
-  h->d_bsum.alloc(2 * nb + 2);
+  h->d_bsum.alloc(nb);
 }
 
 void upload_bcs(mpm_gpu_t h) {
@@ -974,6 +974,7 @@ void refresh_state(mpm_gpu_t h) {
   s.mats_t = h->ntangent > 0 ? h->d_mats_t.p : nullptr;
   s.tpbuf = h->ntangent > 0 ? h->d_tpbuf.p : nullptr;
   s.tangent_mass_floor = h->tangent_mass_floor;
+  s.remove_lost = h->cfg.locate_particles ? 0 : 1;
   s.any_softening = 0;
   for (auto& m : h->mats) s.any_softening |= (m.type == 1 && m.softening) ? 1 : 0;
   s.plist = h->any_mc ? h->d_plist.p : nullptr;
@@ -2933,7 +2934,7 @@ int mpm_gpu_adjoint_reverse(mpm_gpu_t h, const double* dL_dx, const double* dL_d
         copy_state(h, t, t.seg_pf.p + t.pfc_n * j, t.seg_sv.p + t.sv_n * j, t.seg_cell.p + t.cell_n * j,
                    false);
       set_gravity(h, a, t.step0 + k);
-      h->prof.begin(K_ADJ_RECOMPUTE, h->stream, SORT_KERNELS + 2);
+      h->prof.begin(K_ADJ_RECOMPUTE, h->stream, sort_kernels(h->ds) + 2);
       launch_p2g_nodes_fp64(dim, h->ds, a, h->stream);
       h->prof.end(K_ADJ_RECOMPUTE, h->stream);
       launch_adjoint_step(dim, h->ds, A, a, h->stream, h->prof);

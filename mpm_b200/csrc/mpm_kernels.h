@@ -63,9 +63,16 @@ constexpr int PAD_PARTICLES = 128;
 const char* kernel_name(int kid);
 
 // Counts kernel launches; when enabled, brackets every phase (one kernel, or
-// the SORT_KERNELS kernels of the counting sort) with a pair of CUDA events on
+// the kernels of the counting sort) with a pair of CUDA events on
 // the launching stream and accumulates their elapsed times.
-constexpr int SORT_KERNELS = 5;  // count, two scan levels, scan add, fill
+// The sort is one kernel (a cluster) up to these sizes and five (reset, count,
+// chunk scans, scan add, fill) above.  Measured, a 2D step with one / five: 3,200
+// particles 16.4 / 18.5 us, 8,000 18.5 / 20.6, 16,384 20.5 / 22.6, 32,400 26.6 /
+// 21.0, 65,536 32.8 / 22.6.
+constexpr int64_t SORT_SMALL_NP = 16384, SORT_SMALL_CELLS = 65536;
+inline int sort_kernels(const DevState& s) {
+  return s.np <= SORT_SMALL_NP && s.ncells <= SORT_SMALL_CELLS ? 1 : 5;
+}
 struct Profiler {
   bool enabled = false;
   int64_t launches = 0;
@@ -101,7 +108,8 @@ struct PersistentArgs {
 cudaError_t launch_steps_persistent_mixed(int dim, const DevState& s, const StepArgs& a,
                                           const PersistentArgs& q, cudaStream_t st);
 // shared by both paths: the per-step counting sort and the exhaustive locate
-void counting_sort(const DevState& s, cudaStream_t st);
+// (words: it also resets the step's list lengths, nlost and nplastic)
+void counting_sort(const DevState& s, cudaStream_t st, int words = 0);
 void launch_locate_fallback(int dim, const DevState& s, int remove_lost, cudaStream_t st);
 // PODParticle records (pod_particle.h:12-62): 74 fields, caller's layout
 constexpr int POD_NFIELDS = 74;

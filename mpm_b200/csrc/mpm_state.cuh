@@ -186,6 +186,7 @@ struct DevState {
   float* dndx_cf = nullptr;       // [ncells][NV][DIM]
   const MaterialT<float>* mats_f = nullptr;
 
+  int remove_lost = 0;            // locate_particles false: unlocatable particles are removed
   int any_softening = 0;          // some MohrCoulomb material softens (phi..tc vary)
   // test hook: the staged G2P's first copy wait runs out on purpose (after its
   // copies have landed), exercising the ERR_TIMEOUT path without a fault
