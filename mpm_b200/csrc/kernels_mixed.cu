@@ -33,10 +33,12 @@
 #include "mpm_state.cuh"
 
 #ifndef MPM_MIXED_G2P_MIN_BLOCKS
-// 80 registers: 0.478 -> 0.374 ms (4M, 3D).  7 and 8 blocks (72 / 64 registers, more
-// spills): early steps g2p 0.389 -> 0.377 / 0.379 ms, step at 2000 0.542 -> 0.545 /
-// 0.547 ms (1M column): no net gain over a run.
-#define MPM_MIXED_G2P_MIN_BLOCKS 6
+// 72 registers, hardly a spill on a grid: 2M particles in 3D 6 / 7 / 8 blocks 135 /
+// 129 / 142 us (8 spill); no difference in 2D.
+#define MPM_MIXED_G2P_MIN_BLOCKS 7
+#endif
+#ifndef MPM_MIXED_G2P_GENERAL_MIN_BLOCKS
+#define MPM_MIXED_G2P_GENERAL_MIN_BLOCKS 6  // 80 registers; spills on a general mesh, more with fewer
 #endif
 #ifndef MPM_MIXED_AFFINE_G2P_MIN_BLOCKS
 #define MPM_MIXED_AFFINE_G2P_MIN_BLOCKS 4  // the nodal velocities stay in registers for B
@@ -917,12 +919,17 @@ __global__ void __launch_bounds__(128) k_stress_mixed(DevState s, float dt) {
   stress_update_mixed<DIM>(s, MGlobalRow<DIM>{s, p}, grad, dt);
 }
 
+template <bool BOX>
+constexpr int mixed_g2p_min_blocks() {
+  return BOX ? MPM_MIXED_G2P_MIN_BLOCKS : MPM_MIXED_G2P_GENERAL_MIN_BLOCKS;
+}
+
 // --------------------------------------------------------------------- G2P
 // MUSL (mpm_scheme_musl.tcc:20-35): the kinematics without committing the
 // positions -- the updated ones go to xnext (k_commit_locate_mixed commits them
 // after the second mapping and the stress update), no locate here.
 template <int DIM, bool STRESS, bool FLIP, bool BOX, bool MUSL = false>
-__global__ void __launch_bounds__(128, MPM_MIXED_G2P_MIN_BLOCKS)
+__global__ void __launch_bounds__(128, mixed_g2p_min_blocks<BOX>())
     k_g2p_mixed(DevState s, double dt, float beta) {
   after_previous();
   static_assert(!(MUSL && STRESS), "MUSL updates the stress after its second mapping");
@@ -1268,7 +1275,7 @@ __device__ __forceinline__ void g2p_staged_block_mixed(const DevState& s, double
 }
 
 template <int DIM, bool FLIP, bool BOX>
-__global__ void __launch_bounds__(MSTAGE_T, MPM_MIXED_G2P_MIN_BLOCKS)
+__global__ void __launch_bounds__(MSTAGE_T, mixed_g2p_min_blocks<BOX>())
     k_g2p_mixed_staged(DevState s, double dt, float beta) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ uint64_t bar[2];

@@ -55,20 +55,21 @@ def test_graded_grid(dim, scheme, update):
     so["v"][:, :dim] = v
     o.set(so)
     start = st["cell"].copy()
-    for n in (1, 99):
-        for s in (g, m, o):
-            s.step(n)
-        a, b = g.read(), o.get()
-        assert_parity(a, b, label=f"{dim}D {scheme} {update}")
-    assert np.count_nonzero(a["cell"] != start) > len(start) // 4, "the block was meant to cross cells"
-    if update == "apic":  # its FP32 error is set by nodes that a corner of the block hardly touches
-        return
-    # FP32 rounding of 100 steps.  Fields: at most a few 2^-24 of their scale a step.  Strain: a step adds dt
-    # times velocity differences over a cell, of velocities off by up to 8 * 2^-24 each; stress: that times 3 K.
-    c = m.read()
-    errs = field_errors(c, a, ("x", "u", "v", "F", "volume", "density", "mass"))
-    assert max(errs.values()) < 100 * 4 * 2.0 ** -24, errs
     dx = min(np.diff(np.unique(prob.coords[:, d])).min() for d in range(dim))
-    strain = 100 * 1e-4 * 16 * 2.0 ** -24 * np.abs(a["v"]).max() / dx
-    assert np.abs(c["strain"] - a["strain"]).max() < strain
-    assert np.abs(c["stress"] - a["stress"]).max() < 5e5 / (1 - 2 * 0.3) * strain
+    for n in (1, 100):
+        for s in (g, m, o):
+            s.step(n - (n > 1))
+        a, b, c = g.read(), o.get(), m.read()
+        assert_parity(a, b, label=f"{dim}D {scheme} {update}")
+        # FP32 rounding of n steps.  Fields: at most a few 2^-24 of their scale a step.  Strain: a step adds dt
+        # times velocity differences over a cell, of velocities off by up to 8 * 2^-24 each; stress: that times 3 K.
+        # Later steps only where the velocities of nodes that a corner of the block hardly touches (FP32
+        # momentum over a tiny mass) do not stay in the particles' velocities, as they do in FLIP and APIC.
+        if n > 1 and scheme == "usl":
+            continue
+        errs = field_errors(c, a, ("x", "u", "v", "F", "volume", "density", "mass"))
+        assert max(errs.values()) < n * 8 * 2.0 ** -24, errs
+        strain = n * 1e-4 * 16 * 2.0 ** -24 * np.abs(a["v"]).max() / dx
+        assert np.abs(c["strain"] - a["strain"]).max() < strain
+        assert np.abs(c["stress"] - a["stress"]).max() < 5e5 / (1 - 2 * 0.3) * strain
+    assert np.count_nonzero(a["cell"] != start) > len(start) // 4, "the block was meant to cross cells"
