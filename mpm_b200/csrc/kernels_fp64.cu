@@ -42,13 +42,13 @@ namespace mpm_b200 {
 namespace {
 
 // ------------------------------------------------------------ counting sort
-// The counts (and, with words, the step's list lengths) set to zero.
+// The counts (and, with words, the length of the list of lost particles) set to zero.
 __global__ void __launch_bounds__(256) k_sort_reset(DevState s, int words) {
   after_previous();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < s.ncells;
        i += (int64_t)gridDim.x * blockDim.x)
     s.cnt[i] = 0;
-  if (words && blockIdx.x == 0 && threadIdx.x == 0) *s.nlost = *s.nplastic = *s.nplastic_heavy = 0;
+  if (words && blockIdx.x == 0 && threadIdx.x == 0) *s.nlost = 0;
 }
 
 __global__ void __launch_bounds__(256) k_count(DevState s) {
@@ -139,7 +139,7 @@ __global__ void __cluster_dims__(SORT_CLUSTER, 1, 1) __launch_bounds__(1024) k_s
   const int r = (int)blockIdx.x, first = r * 1024 + (int)threadIdx.x;
   const int nc = (int)s.ncells, np = (int)s.np;
   for (int i = first; i < nc; i += NT) s.cnt[i] = 0;
-  if (words && first == 0) *s.nlost = *s.nplastic = *s.nplastic_heavy = 0;
+  if (words && first == 0) *s.nlost = 0;
   cl.sync();
   for (int p = first; p - (int)(threadIdx.x & 31) < np; p += NT) count_particle(s, p);  // whole warps
   cl.sync();
@@ -429,6 +429,7 @@ __device__ __forceinline__ void node_accel_update(const DevState& s, double m, c
 template <int DIM, int MODE>
 __global__ void __launch_bounds__(256) k_nodes(DevState s, double dt, double damping) {
   after_previous();
+  if (MODE != 2 && blockIdx.x == 0 && threadIdx.x == 0) *s.nplastic = *s.nplastic_heavy = 0;
   const int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= s.nn) return;
   const int64_t nn = s.nn;
@@ -1074,7 +1075,7 @@ __global__ void k_locate_fallback(DevState s, int remove_lost) {
 
 inline unsigned nblocks(int64_t n, int threads) { return (unsigned)((n + threads - 1) / threads); }
 
-// words: also reset the step's list lengths.  One cluster takes the sort of up
+// words: also reset the length of the list of lost particles.  One cluster takes the sort of up
 // to SORT_SMALL_NP particles and SORT_SMALL_CELLS cells.
 void counting_sort_impl(const DevState& s, cudaStream_t st, int words) {
   const int64_t nc = s.ncells;
@@ -1104,22 +1105,28 @@ void prefer_shared_memory() {
   }
 }
 
+// The plastic returns of a step.
+template <int DIM>
+void returns_fp64(const DevState& s, const StepArgs& a, cudaStream_t st, Profiler& pr) {
+  if (!s.sv) return;
+  const unsigned all = nblocks(s.np, 128), cap = 148u * (unsigned)return_blocks(a);
+  pr.begin(K_MC_RETURN, st);
+  // A plain launch: the return keeps part of its state in local memory and needs
+  // the L1 that the staged G2P gave to shared memory.  Blocks that an SM takes
+  // on while G2P's last ones run keep that split to their end: a flowing 0.8M-
+  // particle step took 323 us with a dependent launch here, 263 with this one.
+  k_mc_return<DIM><<<all < cap ? all : cap, 128, 0, st>>>(s);
+  pr.end(K_MC_RETURN, st);
+}
+
 template <int DIM, bool BOX>
 void step_impl(const DevState& s, const StepArgs& a, cudaStream_t st, Profiler& pr) {
   const int64_t np = s.np, nn = s.nn;
   if (np == 0) return;
   const unsigned nt = (unsigned)node_block(a);
   const unsigned pb128 = nblocks(np, 128), nb = nblocks(nn, nt);
-  const unsigned mcb = (unsigned)std::min<int64_t>(nblocks(np, 128), 148 * return_blocks(a));
   auto mc_returns = [&]() {
-    if (!s.sv) return;
-    pr.begin(K_MC_RETURN, st);
-    // A plain launch: the return keeps part of its state in local memory and needs
-    // the L1 that the staged G2P gave to shared memory.  Blocks that an SM takes
-    // on while G2P's last ones run keep that split to their end: a flowing 0.8M-
-    // particle step took 323 us with a dependent launch here, 263 with this one.
-    k_mc_return<DIM><<<mcb, 128, 0, st>>>(s);
-    pr.end(K_MC_RETURN, st);
+    if (!a.defer_returns) returns_fp64<DIM>(s, a, st, pr);
   };
   auto p2g = [&](auto mode) {
     constexpr int MODE = decltype(mode)::value;
@@ -1127,9 +1134,9 @@ void step_impl(const DevState& s, const StepArgs& a, cudaStream_t st, Profiler& 
       constexpr int AFF = decltype(aff)::value;
       constexpr int TT = p2g_tile_t<BOX, AFF>();
       if (BOX && !AFF && tile_threads(a, BOX) == 128)
-        launch_dependent(k_p2g_tiles<DIM, MODE, BOX, AFF, 128>, nblocks(s.ncells, 128 / Elem<DIM>::NV), 128, 0, st, s, a.g[0], a.g[1], a.g[2]);
+        launch_kernel(!a.returns_first, k_p2g_tiles<DIM, MODE, BOX, AFF, 128>, nblocks(s.ncells, 128 / Elem<DIM>::NV), 128, 0, st, s, a.g[0], a.g[1], a.g[2]);
       else
-        launch_dependent(k_p2g_tiles<DIM, MODE, BOX, AFF>, nblocks(s.ncells, TT / Elem<DIM>::NV), TT, 0, st, s, a.g[0], a.g[1], a.g[2]);
+        launch_kernel(!a.returns_first, k_p2g_tiles<DIM, MODE, BOX, AFF>, nblocks(s.ncells, TT / Elem<DIM>::NV), TT, 0, st, s, a.g[0], a.g[1], a.g[2]);
     };
     if constexpr (MODE != 1) {  // the mass-momentum mapping velocity
       if (a.vupd == 2 || a.vupd == 4) return launch(std::integral_constant<int, 1>{});
@@ -1150,9 +1157,14 @@ void step_impl(const DevState& s, const StepArgs& a, cudaStream_t st, Profiler& 
     }
   };
   if (a.scheme == 1 && a.phase == 2) goto usl_second_half;
+  if (a.returns_first) {
+    fork_side(a, st);
+    returns_fp64<DIM>(s, a, a.side, pr);
+  }
   pr.begin(K_SORT, st, sort_kernels(s));
   counting_sort_impl(s, st, 1);
   pr.end(K_SORT, st);
+  if (a.returns_first) join_side(a, st);
   if (a.scheme == 2) {  // MUSL (mpm_scheme_musl.tcc)
     pr.begin(K_P2G, st);
     p2g(std::integral_constant<int, 2>{});
@@ -1254,6 +1266,10 @@ __global__ void k_material_batch(int64_t n, MaterialParams m, const double* stre
 }
 
 }  // namespace
+
+void launch_returns_fp64(int dim, const DevState& s, const StepArgs& a, cudaStream_t st, Profiler& prof) {
+  dim == 2 ? returns_fp64<2>(s, a, st, prof) : returns_fp64<3>(s, a, st, prof);
+}
 
 void launch_step_fp64(int dim, const DevState& s, const StepArgs& a, cudaStream_t st,
                       Profiler& prof) {

@@ -552,6 +552,7 @@ template <int DIM, int MODE>
 __global__ void __launch_bounds__(256, MPM_MIXED_NODES_MIN_BLOCKS) k_nodes_mixed(DevState s, double dt, double damping, double g0,
                                                         double g1, double g2) {
   after_previous();
+  if (MODE != 2 && blockIdx.x == 0 && threadIdx.x == 0) *s.nplastic = *s.nplastic_heavy = 0;
   const double g[3] = {g0, g1, g2};
   node_update_mixed<DIM, MODE>(s, dt, damping, g, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
 }
@@ -1511,32 +1512,44 @@ cudaError_t launch_persistent(const DevState& s, const StepArgs& a, const Persis
                                      args, sm, st);
 }
 
+// The plastic returns of a step.
+template <int DIM>
+void returns_mixed(const DevState& s, const StepArgs& a, cudaStream_t st, Profiler& pr) {
+  if (!s.svf) return;
+  const unsigned all = nblk(s.np, 128), cap = 148u * (unsigned)return_blocks(a);
+  pr.begin(K_MC_RETURN, st);
+  // A plain launch: the return keeps part of its state in local memory and needs
+  // the L1 that the staged G2P gave to shared memory.  Blocks that an SM takes
+  // on while G2P's last ones run keep that split to their end: a flowing 0.8M-
+  // particle step took 323 us with a dependent launch here, 263 with this one.
+  k_mc_return_mixed<DIM><<<all < cap ? all : cap, 128, 0, st>>>(s);
+  pr.end(K_MC_RETURN, st);
+}
+
 template <int DIM, bool BOX>
 void step_mixed(const DevState& s, const StepArgs& a, cudaStream_t st, Profiler& pr) {
   const int64_t np = s.np, nn = s.nn;
   if (np == 0) return;
   const unsigned nt = (unsigned)node_block(a);
   const unsigned pb = nblk(np, 128), nb = nblk(nn, nt);
-  const unsigned mcap = 148u * (unsigned)return_blocks(a);
-  const unsigned mcb = pb < mcap ? pb : mcap;
   // P2G cell tiles of the step's launch shape
   auto p2g = [&](auto mode) {
     constexpr int MODE = decltype(mode)::value;
     constexpr int NV = Elem<DIM>::NV;
     if constexpr (MODE != 1) {  // the mass-momentum mapping velocity (128-thread tiles)
       if (a.vupd == 2 || a.vupd == 4) {
-        launch_dependent(k_p2g_tiles_mixed<DIM, MODE, BOX, 128, 1>, nblk(s.ncells, 128 / NV), 128, 0, st, s);
+        launch_kernel(!a.returns_first, k_p2g_tiles_mixed<DIM, MODE, BOX, 128, 1>, nblk(s.ncells, 128 / NV), 128, 0, st, s);
         return;
       }
       if (a.vupd == 3) {
-        launch_dependent(k_p2g_tiles_mixed<DIM, MODE, BOX, 128, 2>, nblk(s.ncells, 128 / NV), 128, 0, st, s);
+        launch_kernel(!a.returns_first, k_p2g_tiles_mixed<DIM, MODE, BOX, 128, 2>, nblk(s.ncells, 128 / NV), 128, 0, st, s);
         return;
       }
     }
     if (BOX && tile_threads(a, BOX) == 128)
-      launch_dependent(k_p2g_tiles_mixed<DIM, MODE, BOX, 128>, nblk(s.ncells, 128 / NV), 128, 0, st, s);
+      launch_kernel(!a.returns_first, k_p2g_tiles_mixed<DIM, MODE, BOX, 128>, nblk(s.ncells, 128 / NV), 128, 0, st, s);
     else
-      launch_dependent(k_p2g_tiles_mixed<DIM, MODE, BOX>, nblk(s.ncells, p2g_tile_t<BOX>() / NV),
+      launch_kernel(!a.returns_first, k_p2g_tiles_mixed<DIM, MODE, BOX>, nblk(s.ncells, p2g_tile_t<BOX>() / NV),
                        p2g_tile_t<BOX>(), 0, st, s);
   };
   // G2P of the mapping-matrix updates (ASFLIP 2, TPIC 3, APIC 4)
@@ -1551,19 +1564,17 @@ void step_mixed(const DevState& s, const StepArgs& a, cudaStream_t st, Profiler&
       launch_dependent(k_g2p_mixed_affine<DIM, STRESS, 4, BOX>, pb, 128, 0, st, s, a.dt, b);
   };
   auto mc_returns = [&]() {
-    if (!s.svf) return;
-    pr.begin(K_MC_RETURN, st);
-    // A plain launch: the return keeps part of its state in local memory and needs
-    // the L1 that the staged G2P gave to shared memory.  Blocks that an SM takes
-    // on while G2P's last ones run keep that split to their end: a flowing 0.8M-
-    // particle step took 323 us with a dependent launch here, 263 with this one.
-    k_mc_return_mixed<DIM><<<mcb, 128, 0, st>>>(s);
-    pr.end(K_MC_RETURN, st);
+    if (!a.defer_returns) returns_mixed<DIM>(s, a, st, pr);
   };
   if (a.scheme == 1 && a.phase == 2) goto usl_second_half;
+  if (a.returns_first) {
+    fork_side(a, st);
+    returns_mixed<DIM>(s, a, a.side, pr);
+  }
   pr.begin(K_SORT, st, sort_kernels(s));
   counting_sort(s, st, 1);
   pr.end(K_SORT, st);
+  if (a.returns_first) join_side(a, st);
   if (a.scheme == 2) {  // MUSL (mpm_scheme_musl.tcc:20-35)
     pr.begin(K_P2G, st);
     p2g(std::integral_constant<int, 2>{});
@@ -1655,6 +1666,10 @@ cudaError_t launch_steps_persistent_mixed(int dim, const DevState& s, const Step
   if (dim == 2)
     return a.flip ? launch_persistent<2, true>(s, a, q, st) : launch_persistent<2, false>(s, a, q, st);
   return a.flip ? launch_persistent<3, true>(s, a, q, st) : launch_persistent<3, false>(s, a, q, st);
+}
+
+void launch_returns_mixed(int dim, const DevState& s, const StepArgs& a, cudaStream_t st, Profiler& prof) {
+  dim == 2 ? returns_mixed<2>(s, a, st, prof) : returns_mixed<3>(s, a, st, prof);
 }
 
 void launch_step_mixed(int dim, const DevState& s, const StepArgs& a, cudaStream_t st,

@@ -385,6 +385,9 @@ struct mpm_gpu_solver {
   size_t h_rows_n = 0;
   size_t h_stage_bytes = 0;
   cudaEvent_t stage_ev[2] = {nullptr, nullptr};
+  // a step's plastic returns beside the next one's sort (StepArgs::returns_first)
+  cudaStream_t side = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
 
   // launch shape of the value steps (mpm_gpu_set_launch_shape, mpm_gpu_autotune);
   // zeros are the built-in defaults
@@ -1374,8 +1377,11 @@ int mpm_gpu_create(const mpm_gpu_config* cfg, mpm_gpu_t* out) {
   // runs out on purpose, so the MPM_ERR_TIMEOUT path can be exercised
   if (const char* e = std::getenv("MPM_B200_TEST_WAIT_TIMEOUT")) h->ds.test_wait_timeout = std::atoi(e) != 0;
   if (cudaSetDevice(cfg->device) != cudaSuccess ||
-      cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess) {
-    delete h;
+      cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaEventCreateWithFlags(&h->fork, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&h->join, cudaEventDisableTiming) != cudaSuccess) {
+    mpm_gpu_destroy(h);
     return MPM_ERR_CUDA;
   }
   *out = h;
@@ -1389,6 +1395,9 @@ int mpm_gpu_destroy(mpm_gpu_t h) {
     cudaStreamSynchronize(h->stream);
     cudaStreamDestroy(h->stream);
   }
+  if (h->side) cudaStreamDestroy(h->side);
+  if (h->fork) cudaEventDestroy(h->fork);
+  if (h->join) cudaEventDestroy(h->join);
   if (h->h_stage) cudaFreeHost(h->h_stage);
   if (h->h_rows) cudaFreeHost(h->h_rows);
   for (auto& e : h->stage_ev)
@@ -1769,7 +1778,8 @@ static bool same_step(const DevState& a, const DevState& b, const StepArgs& x, c
          x.remove_lost == y.remove_lost && x.dt == y.dt && x.beta == y.beta &&
          x.damping == y.damping && x.g[0] == y.g[0] && x.g[1] == y.g[1] && x.g[2] == y.g[2] &&
          x.p2g_tile == y.p2g_tile && x.node_threads == y.node_threads &&
-         x.return_blocks_per_sm == y.return_blocks_per_sm;
+         x.return_blocks_per_sm == y.return_blocks_per_sm &&
+         x.defer_returns == y.defer_returns && x.returns_first == y.returns_first;
 }
 
 // The step arguments of the solver's configuration and launch shape (gravity
@@ -1786,6 +1796,9 @@ static StepArgs base_step_args(mpm_gpu_t h) {
   a.p2g_tile = h->shape_p2g_tile;
   a.node_threads = h->shape_node_threads;
   a.return_blocks_per_sm = h->shape_return_bps;
+  a.side = h->side;
+  a.fork = h->fork;
+  a.join = h->join;
   return a;
 }
 
@@ -1871,7 +1884,12 @@ static int run_steps(mpm_gpu_t h, int64_t nsteps, double* elapsed_ms) {
   // launches).  The first step of a call runs eagerly (it sets the kernels'
   // shared-memory attributes outside any capture); profiling runs eagerly.
   bool eager_done = false;
+  // Each step's plastic returns run beside the next step's sort; the call's last
+  // ones after its last step.
+  const bool beside = nsteps > 1 && a.scheme == 1 && h->any_mc && h->ntangent == 0 && !h->prof.enabled;
+  a.defer_returns = beside ? 1 : 0;
   for (int64_t s = 0; s < nsteps; ++s) {
+    a.returns_first = beside && s > 0 ? 1 : 0;
     double gm = 1.0;  // mpm_explicit.tcc:145-153
     if (h->cfg.gravity_ramping_time > 0.0)
       gm = std::min(1.0, static_cast<double>(h->step) * h->cfg.dt / h->cfg.gravity_ramping_time);
@@ -1911,6 +1929,13 @@ static int run_steps(mpm_gpu_t h, int64_t nsteps, double* elapsed_ms) {
     }
     ck(cudaGetLastError(), "kernel launch");
     ++h->step;
+  }
+  if (beside) {
+    if (h->mixed)
+      launch_returns_mixed(h->dim, h->ds, a, h->stream, h->prof);
+    else
+      launch_returns_fp64(h->dim, h->ds, a, h->stream, h->prof);
+    ck(cudaGetLastError(), "kernel launch");
   }
   if (elapsed_ms) ck(cudaEventRecord(e1, h->stream), "cudaEventRecord");
   unsigned words[2] = {0, 0};

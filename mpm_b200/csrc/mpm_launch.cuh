@@ -23,9 +23,10 @@ __device__ __forceinline__ void after_previous() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// (dependent false: a plain launch, for a kernel that also waits on another stream)
 template <class... P, class... A>
-inline void launch_dependent(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem,
-                             cudaStream_t st, const A&... args) {
+inline void launch_kernel(bool dependent, void (*kernel)(P...), unsigned grid, unsigned block,
+                          size_t smem, cudaStream_t st, const A&... args) {
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
@@ -35,8 +36,13 @@ inline void launch_dependent(void (*kernel)(P...), unsigned grid, unsigned block
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = dependent ? 1 : 0;
   cudaLaunchKernelEx(&cfg, kernel, P(args)...);  // an error stays for the caller's cudaGetLastError
+}
+template <class... P, class... A>
+inline void launch_dependent(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem,
+                             cudaStream_t st, const A&... args) {
+  launch_kernel(true, kernel, grid, block, smem, st, args...);
 }
 
 }  // namespace mpm_b200
