@@ -228,7 +228,13 @@ __global__ void __launch_bounds__(T, (tile_min_blocks<BOX, AFF, T>()))
     if (a1 > a0) box_map = cell_map<DIM, true, double>(s, (int)c, nullptr, nullptr);
   }
   double xk[DIM];  // this slot's node, for the branch vectors of the mapping velocity
-  if constexpr (MM && AFF) {
+  if constexpr (MM && AFF && BOX) {
+    int ijk[3] = {0, 0, 0};
+    if (a1 > a0) cell_ijk<DIM>(s, (int)c, ijk);
+    const int off[3] = {off_i(k), off_j(k), off_k(k)};
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) xk[d] = __ldg(&s.axis[d][ijk[d] + off[d]]);
+  } else if constexpr (MM && AFF) {
     int nid[NV];
     double X[NV * DIM];
     if (a1 > a0) cell_nodes_coords<DIM>(s, (int)c, nid, X);
@@ -252,7 +258,7 @@ __global__ void __launch_bounds__(T, (tile_min_blocks<BOX, AFF, T>()))
       for (int d = 0; d < DIM; ++d) rows[RW::XI + d][t] = xi[d];
       if constexpr (MM && AFF) {
         double Mv[DIM * DIM];
-        mapping_velocity_matrix<DIM, AFF>(s, p, pc, x, xi, Mv);
+        mapping_velocity_matrix<DIM, AFF, BOX>(s, p, pc, x, xi, Mv);
 #pragma unroll
         for (int d = 0; d < DIM; ++d) rows[RW::XP + d][t] = x[d];
 #pragma unroll

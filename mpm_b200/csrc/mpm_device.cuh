@@ -304,8 +304,10 @@ __device__ __forceinline__ void dn_dx_node(const double* xi, const Map& map, int
 
 // The matrix M of the mapping velocity v + M r_i of particle p in cell c
 // (position x, local coordinates xi): B D^-1 (AFF 1) with the shape tensor
-// D = sum_i N_i r_i r_i^T, or B (AFF 2).
-template <int DIM, int AFF>
+// D = sum_i N_i r_i r_i^T, or B (AFF 2).  In a box cell the sums over the nodes
+// of N_i r_ia vanish, so D is diagonal, with (1 - xi_a^2) (len_a / 2)^2: no sums
+// and no inverse.
+template <int DIM, int AFF, bool BOX>
 __device__ __forceinline__ void mapping_velocity_matrix(const DevState& s, int64_t p, int c,
                                                         const double* x, const double* xi,
                                                         double* M) {
@@ -316,6 +318,16 @@ __device__ __forceinline__ void mapping_velocity_matrix(const DevState& s, int64
   if constexpr (AFF == 2) {
 #pragma unroll
     for (int q = 0; q < DIM * DIM; ++q) M[q] = B[q];
+  } else if constexpr (BOX) {
+    int ijk[3] = {0, 0, 0};
+    cell_ijk<DIM>(s, c, ijk);
+#pragma unroll
+    for (int b = 0; b < DIM; ++b) {
+      const double h = s.axcell[b][ijk[b]].ihl;
+      const double di = h * h / ((1. - xi[b]) * (1. + xi[b]));
+#pragma unroll
+      for (int a = 0; a < DIM; ++a) M[a * DIM + b] = B[a * DIM + b] * di;
+    }
   } else {
     int nid[NV];
     double X[NV * DIM], N[NV], T[DIM * DIM], Ti[DIM * DIM];
