@@ -1380,11 +1380,8 @@ int mpm_gpu_create(const mpm_gpu_config* cfg, mpm_gpu_t* out) {
   // runs out on purpose, so the MPM_ERR_TIMEOUT path can be exercised
   if (const char* e = std::getenv("MPM_B200_TEST_WAIT_TIMEOUT")) h->ds.test_wait_timeout = std::atoi(e) != 0;
   if (cudaSetDevice(cfg->device) != cudaSuccess ||
-      cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaEventCreateWithFlags(&h->fork, cudaEventDisableTiming) != cudaSuccess ||
-      cudaEventCreateWithFlags(&h->join, cudaEventDisableTiming) != cudaSuccess) {
-    mpm_gpu_destroy(h);
+      cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess) {
+    delete h;
     return MPM_ERR_CUDA;
   }
   *out = h;
@@ -1890,6 +1887,14 @@ static int run_steps(mpm_gpu_t h, int64_t nsteps, double* elapsed_ms) {
   // Each step's plastic returns run beside the next step's sort; the call's last
   // ones after its last step.
   const bool beside = nsteps > 1 && a.scheme == 1 && h->any_mc && h->ntangent == 0 && !h->prof.enabled;
+  if (beside && !h->side) {
+    ck(cudaEventCreateWithFlags(&h->fork, cudaEventDisableTiming), "cudaEventCreate");
+    ck(cudaEventCreateWithFlags(&h->join, cudaEventDisableTiming), "cudaEventCreate");
+    ck(cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking), "cudaStreamCreate");
+    a.side = h->side;
+    a.fork = h->fork;
+    a.join = h->join;
+  }
   a.defer_returns = beside ? 1 : 0;
   for (int64_t s = 0; s < nsteps; ++s) {
     a.returns_first = beside && s > 0 ? 1 : 0;
