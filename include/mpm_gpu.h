@@ -22,7 +22,7 @@
  *   particles include/particles/particle.tcc:145-306 particle state (POD)
  *
  * Threading: one host thread per handle.  All device work of a handle runs
- * on its own CUDA stream; mpm_gpu_step() returns once the steps are queued
+ * on its own CUDA streams; mpm_gpu_step() returns once the steps are queued
  * and their error word has been read (it synchronises the stream at the end
  * of the call).
  */
@@ -208,13 +208,13 @@ int mpm_gpu_step_timed(mpm_gpu_t h, int64_t nsteps, double* elapsed_ms);
 /* Launch shape of the steps (no counterpart in the reference, whose steps
  * are host loops): threads of a P2G cell tile on a tensor-product grid (128
  * or 256), threads of a node-kernel block (128 or 256), blocks per SM of the
- * plastic-return kernel (4, 8 or 16); 0 keeps the built-in default (256 up
- * to 100,000 particles and 128 above, 256, 8).  Results do not depend on it.  mpm_gpu_get_launch_shape writes the
- * three values in use.  mpm_gpu_autotune times each candidate over `steps`
- * steps (at least 3, after 2 untimed ones) of the solver's own state, one
- * field at a time, keeps
- * the fastest, and restores the particle state and step counter, so the run
- * then continues exactly as without it; report (report_len bytes, may be
+ * plastic-return kernel (4, 8 or 16); 0 keeps the built-in default (256 up to
+ * 100,000 particles and 128 above, 256, 8).  Results do not depend on it.
+ * mpm_gpu_get_launch_shape writes the three values in use.  mpm_gpu_autotune
+ * times each candidate over `steps` steps (at least 3, after 2 untimed ones)
+ * of the solver's own state, one field at a time, keeps the fastest, and
+ * restores the particle state and step counter, so the run then continues
+ * exactly as without it; report (report_len bytes, may be
  * NULL) receives the per-candidate milliseconds per step as JSON.  It holds a
  * copy of the particle state on the device meanwhile (MPM_ERR_ALLOC if that
  * does not fit).  Not with sensitivities on. */
@@ -227,8 +227,8 @@ int mpm_gpu_autotune(mpm_gpu_t h, int64_t steps, char* report, size_t report_len
  * reference): with steps_per_launch > 0, mpm_gpu_step advances up to that
  * many whole steps per cooperative kernel launch (after the first launch of a
  * call, launches of that many steps replay a captured CUDA graph), every block resident, the
- * passes of a step (sort, P2G, node update, G2P and stress, plastic returns,
- * exhaustive locate) separated by grid barriers with bounded waits
+ * passes of a step (sort, P2G, node update, G2P with stress and locate, plastic
+ * returns) separated by grid barriers with bounded waits
  * (MPM_ERR_TIMEOUT when one runs out); 0 returns to one launch per pass,
  * replayed from a CUDA graph (the default).  Results are bit for bit those
  * of the per-pass launches.  Mixed precision, USL, FLIP or PIC, on a
