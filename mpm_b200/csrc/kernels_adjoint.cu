@@ -119,7 +119,7 @@ __device__ __forceinline__ void strain_rates(const DevState& s, int c, const Box
                                              double* sr, bool* sr_live, double* src, bool* src_live) {
   constexpr int NV = Elem<DIM>::NV;
   const int64_t nn = s.nn;
-  const CentroidGrad<DIM, true> Dc(s, c);
+  const double* Dc = s.dndx_c + (int64_t)c * NV * DIM;
 #pragma unroll
   for (int k = 0; k < 6; ++k) sr[k] = 0.;
 #pragma unroll
@@ -134,7 +134,7 @@ __device__ __forceinline__ void strain_rates(const DevState& s, int c, const Box
     for (int d = 0; d < DIM; ++d) Dn[d] = G[d] * b.ihl[d];
     double dc[DIM];
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) dc[d] = Dc.at(i, d);
+    for (int d = 0; d < DIM; ++d) dc[d] = Dc[i * DIM + d];
     if constexpr (DIM == 2) {
       sr[0] += Dn[0] * vel[0];
       sr[1] += Dn[1] * vel[1];
@@ -452,11 +452,10 @@ __global__ void __launch_bounds__(256) k_adj_scatter(DevState s, AdjointArgs A) 
   if (a1 > a0) {
     int ijk[3] = {0, 0, 0};
     cell_ijk<DIM>(s, (int)c, ijk);
-    const CentroidGrad<DIM, true> Dc(s, (int)c);
 #pragma unroll
     for (int d = 0; d < DIM; ++d) {
       ihl[d] = s.axcell[d][ijk[d]].ihl;
-      dc[d] = Dc.at(k, d);
+      dc[d] = s.dndx_c[((int64_t)c * NV + k) * DIM + d];
     }
   }
   const int64_t np = s.np;

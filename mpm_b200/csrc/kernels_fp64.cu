@@ -504,13 +504,13 @@ struct SmemRow {
 // mpm_scheme.tcc:75-103: F increment (particle.tcc:1580-1628), strain
 // (:819-876), volume (:598-605), material stress (:880-889), F (:1654-1658).
 // D: dN/dx at the particle (start of step); the cell's centroid gradients
-// come from the axis tables or the per-cell table (CentroidGrad).
-template <int DIM, bool BOX, class Row>
+// come from the per-cell table computed once from the mesh.
+template <int DIM, class Row>
 __device__ __forceinline__ void stress_update(const DevState& s, const Row& r, int c,
                                               const int* nid, const double* D, double dt) {
   constexpr int NV = Elem<DIM>::NV;
   const int64_t nn = s.nn;
-  const CentroidGrad<DIM, BOX> Dc(s, c);
+  const double* Dc = s.dndx_c + (int64_t)c * NV * DIM;
   double Fi[DIM * DIM];
 #pragma unroll
   for (int r = 0; r < DIM; ++r)
@@ -530,7 +530,7 @@ __device__ __forceinline__ void stress_update(const DevState& s, const Row& r, i
     const double* Dn = &D[i * DIM];
     double dc[DIM];
 #pragma unroll
-    for (int d = 0; d < DIM; ++d) dc[d] = Dc.at(i, d);
+    for (int d = 0; d < DIM; ++d) dc[d] = __ldg(&Dc[i * DIM + d]);
     if constexpr (DIM == 2) {
       sr[0] += Dn[0] * vel[0];
       sr[1] += Dn[1] * vel[1];
@@ -664,7 +664,7 @@ __global__ void __launch_bounds__(128) k_stress(DevState s, double dt) {
   particle_xi<DIM, BOX>(s, c, x, xi);
   cell_nodes_for<DIM, BOX>(s, c, nid, X);
   dn_dx_all<DIM, BOX>(s, c, xi, X, D);
-  stress_update<DIM, BOX>(s, GlobalRow{s, p}, c, nid, D, dt);
+  stress_update<DIM>(s, GlobalRow{s, p}, c, nid, D, dt);
 }
 
 // --------------------------------------------------------------------- G2P
@@ -811,7 +811,7 @@ __global__ void __launch_bounds__(128, MPM_G2P_MIN_BLOCKS) k_g2p(DevState s, dou
   if constexpr (STRESS) {
     double D[NV * DIM];
     dn_dx_all<DIM, BOX>(s, c, xi, X, D);
-    stress_update<DIM, BOX>(s, GlobalRow{s, p}, c, nid, D, dt);
+    stress_update<DIM>(s, GlobalRow{s, p}, c, nid, D, dt);
   }
   settle_particle<DIM, BOX>(s, p, xn, c);
 }
@@ -933,7 +933,7 @@ __global__ void __launch_bounds__(STAGE_T, MPM_G2P_MIN_BLOCKS)
     int nid[NV];
     cell_nodes_for<DIM, BOX>(s, c, nid, X);
     dn_dx_all<DIM, BOX>(s, c, xi, X, D);
-    stress_update<DIM, BOX>(s, r, c, nid, D, dt);
+    stress_update<DIM>(s, r, c, nid, D, dt);
   }
   bulk::fence_shared_to_async();
   __syncthreads();

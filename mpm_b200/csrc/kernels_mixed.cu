@@ -141,11 +141,16 @@ __device__ __forceinline__ void xi_f32(const DevState& s, int c, const double* x
   for (int d = 0; d < DIM; ++d) xf[d] = (float)xi[d];
 }
 
-// node ids and nodal coordinates relative to node 0 of the cell (FP32) of a
-// general mesh
-template <int DIM>
+// node ids and nodal coordinates relative to node 0 of the cell (FP32); the
+// coordinates are not needed (nor set) for the box cells of a tensor-product
+// grid
+template <int DIM, bool BOX>
 __device__ __forceinline__ void cell_nodes_rel(const DevState& s, int c, int* nid, float* Xr) {
   constexpr int NV = Elem<DIM>::NV;
+  if constexpr (BOX) {
+    grid_cell_nodes<DIM>(s, c, nid);
+    return;
+  }
   double X[NV * DIM];
   cell_nodes_coords<DIM>(s, c, nid, X);
 #pragma unroll
@@ -264,7 +269,7 @@ __device__ __forceinline__ void p2g_tile_mixed(const DevState& s, int64_t bx) {
       if constexpr (!BOX) {
         int nid[NV];
         float Xr[NV * DIM];
-        cell_nodes_rel<DIM>(s, pc, nid, Xr);
+        cell_nodes_rel<DIM, false>(s, pc, nid, Xr);
         const CellMap<DIM, false, float> m = cell_map<DIM, false>(s, pc, &v[RW::XI], Xr);
 #pragma unroll
         for (int q = 0; q < DIM * DIM; ++q) v[RW::INV + q] = m.inv[q];
@@ -861,11 +866,11 @@ __device__ __forceinline__ void stress_update_mixed(const DevState& s, const Row
   }
 }
 
-template <int DIM>
+template <int DIM, bool BOX>
 __device__ __forceinline__ void dn_dx_all_f(const DevState& s, int c, const float* xi,
                                             const float* Xr, float* D) {
   constexpr int NV = Elem<DIM>::NV;
-  const CellMap<DIM, false, float> map = cell_map<DIM, false>(s, c, xi, Xr);
+  const CellMap<DIM, BOX, float> map = cell_map<DIM, BOX>(s, c, xi, Xr);
   float G[NV * DIM];
   grad_shapefn<DIM>(xi, G);
 #pragma unroll
@@ -889,7 +894,7 @@ __device__ __forceinline__ void gather_particle(const DevState& s, int c, const 
     int nid[NV];
     xi_f32<DIM, false>(s, c, x, xi);
     shapefn<DIM>(xi, N);
-    cell_nodes_rel<DIM>(s, c, nid, Xr);
+    cell_nodes_rel<DIM, false>(s, c, nid, Xr);
 #pragma unroll
     for (int d = 0; d < DIM; ++d) {
       nvel[d] = 0.f;
@@ -907,7 +912,7 @@ __device__ __forceinline__ void gather_particle(const DevState& s, int c, const 
     }
     if constexpr (GRAD) {
       float D[NV * DIM];
-      dn_dx_all_f<DIM>(s, c, xi, Xr, D);
+      dn_dx_all_f<DIM, false>(s, c, xi, Xr, D);
       *grad = velocity_gradient<DIM>(s, c, nid, D);
     }
   }
@@ -1063,7 +1068,7 @@ __global__ void __launch_bounds__(128, BOX ? 6 : MPM_MIXED_AFFINE_G2P_MIN_BLOCKS
     }
     float D[NV * DIM];
     if constexpr (TPIC || ASFLIP || STRESS) {
-      dn_dx_all_f<DIM>(s, c, xi, Xr, D);
+      dn_dx_all_f<DIM, BOX>(s, c, xi, Xr, D);
       grad = velocity_gradient<DIM>(s, c, nid, D);
     }
 #pragma unroll

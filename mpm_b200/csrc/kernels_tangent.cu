@@ -395,7 +395,7 @@ __global__ void __launch_bounds__(128, MPM_TANGENT_G2P_MIN_BLOCKS) k_stress_tang
   } else {
     jinv_dual<DIM>(xi, X, inv);
   }
-  const CentroidGrad<DIM, BOX> Dc(s, c);
+  const double* Dc = s.dndx_c + (int64_t)c * NV * DIM;
   D Fi[DIM * DIM];
 #pragma unroll
   for (int r = 0; r < DIM; ++r) Fi[r * DIM + r] = D(1.);
@@ -416,8 +416,8 @@ __global__ void __launch_bounds__(128, MPM_TANGENT_G2P_MIN_BLOCKS) k_stress_tang
       sr[0] += Dn[0] * vel[0];
       sr[1] += Dn[1] * vel[1];
       sr[3] += Dn[1] * vel[0] + Dn[0] * vel[1];
-      src[0] += Dc.at(i, 0) * vel[0];
-      src[1] += Dc.at(i, 1) * vel[1];
+      src[0] += Dc[i * DIM + 0] * vel[0];
+      src[1] += Dc[i * DIM + 1] * vel[1];
     } else {
       sr[0] += Dn[0] * vel[0];
       sr[1] += Dn[1] * vel[1];
@@ -425,9 +425,9 @@ __global__ void __launch_bounds__(128, MPM_TANGENT_G2P_MIN_BLOCKS) k_stress_tang
       sr[3] += Dn[1] * vel[0] + Dn[0] * vel[1];
       sr[4] += Dn[2] * vel[1] + Dn[1] * vel[2];
       sr[5] += Dn[2] * vel[0] + Dn[0] * vel[2];
-      src[0] += Dc.at(i, 0) * vel[0];
-      src[1] += Dc.at(i, 1) * vel[1];
-      src[2] += Dc.at(i, 2) * vel[2];
+      src[0] += Dc[i * DIM + 0] * vel[0];
+      src[1] += Dc[i * DIM + 1] * vel[1];
+      src[2] += Dc[i * DIM + 2] * vel[2];
     }
   }
 #pragma unroll

@@ -284,33 +284,6 @@ __device__ __forceinline__ CellMap<DIM, BOX, R> cell_map(const DevState& s, int 
   return m;
 }
 
-// dN_i/dx of local node i at the centroid of cell c (the volume update's,
-// cell.tcc:33-65): on a box +-(1 / NV) 2 / len from the axis tables, elsewhere
-// from the per-cell table, 192 bytes a cell in 3D (24 loads a particle: staged
-// FP64 G2P of 256k particles 54 -> 50 us without).
-template <int DIM, bool BOX>
-struct CentroidGrad {
-  double h[DIM];
-  const double* row;
-  __device__ __forceinline__ CentroidGrad(const DevState& s, int c) {
-    constexpr int NV = Elem<DIM>::NV;
-    if constexpr (BOX) {
-      int ijk[3] = {0, 0, 0};
-      cell_ijk<DIM>(s, c, ijk);
-#pragma unroll
-      for (int d = 0; d < DIM; ++d) h[d] = (1. / NV) * __ldg(&s.axcell[d][ijk[d]].ihl);
-    } else {
-      row = s.dndx_c + (int64_t)c * NV * DIM;
-    }
-  }
-  __device__ __forceinline__ double at(int i, int d) const {
-    if constexpr (BOX)
-      return (d == 0 ? off_i(i) : (d == 1 ? off_j(i) : off_k(i))) ? h[d] : -h[d];
-    else
-      return __ldg(&row[i * DIM + d]);
-  }
-};
-
 // node ids of cell c and, off a tensor-product grid, its nodal coordinates
 template <int DIM, bool BOX>
 __device__ __forceinline__ void cell_nodes_for(const DevState& s, int c, int* nid, double* X) {

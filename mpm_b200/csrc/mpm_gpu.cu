@@ -770,18 +770,15 @@ void upload_mesh(mpm_gpu_t h) {
       h->d_axcell[d].upload(h->axcell[d].data(), h->axcell[d].size(), st);
     }
   if (h->mixed) {
+    std::vector<float> f(h->dndx_c.begin(), h->dndx_c.end());
+    h->d_dndx_cf.upload(f.data(), f.size(), st);
     h->d_nfv.alloc((size_t)nfv_stride(dim) * h->nnodes);
     ck(cudaMemsetAsync(h->d_nfv.p, 0, sizeof(float) * nfv_stride(dim) * h->nnodes, st), "memset");
+    ck(cudaStreamSynchronize(st), "sync");  // f is a stack temporary
+  } else {
+    h->d_dndx_c.upload(h->dndx_c.data(), h->dndx_c.size(), st);
   }
   if (!h->structured) {
-    std::vector<float> f;
-    if (h->mixed) {
-      f.assign(h->dndx_c.begin(), h->dndx_c.end());
-      h->d_dndx_cf.upload(f.data(), f.size(), st);
-    } else {
-      h->d_dndx_c.upload(h->dndx_c.data(), h->dndx_c.size(), st);
-    }
-    ck(cudaStreamSynchronize(st), "sync");  // f is a stack temporary
     h->d_nc_off.upload(h->nc_off.data(), h->nc_off.size(), st);
     h->d_nc_cell.alloc(std::max<size_t>(1, h->nc_cell.size()));
     h->d_nc_cell.upload(h->nc_cell.data(), h->nc_cell.size(), st);
@@ -1437,6 +1434,19 @@ int mpm_gpu_set_mesh(mpm_gpu_t h, int64_t nnodes, const double* coords, int64_t 
     cell_geometry(dim, X.data(), &h->geom[c], &h->cell_volume[c]);
     if (!(h->cell_volume[c] > 0)) throw InvalidArg("Negative or zero volume cell, misconfigured cell!");
   }
+  // dN/dx at the cell centroid (cell.tcc:33-65), once per cell
+  h->dndx_c.resize((size_t)ncells * nv * dim);
+  for (int64_t c = 0; c < ncells; ++c) {
+    for (int i = 0; i < nv; ++i) {
+      const int64_t n = cell_nodes[c * nv + i];
+      for (int d = 0; d < dim; ++d) X[i * dim + d] = coords[n * dim + d];
+    }
+    double xi0[3] = {0., 0., 0.};
+    if (dim == 2)
+      dn_dx<2>(xi0, X.data(), &h->dndx_c[(size_t)c * nv * dim]);
+    else
+      dn_dx<3>(xi0, X.data(), &h->dndx_c[(size_t)c * nv * dim]);
+  }
   // A tensor-product grid needs no connectivity tables: node ids, neighbours
   // and the cells around a node follow from (i, j, k).
   h->structured = detect_structured(h);
@@ -1452,19 +1462,6 @@ int mpm_gpu_set_mesh(mpm_gpu_t h, int64_t nnodes, const double* coords, int64_t 
     upload_bcs(h);  // every node gets a (possibly empty) constraint slot
     h->mesh_set = true;
     return MPM_OK;
-  }
-  // dN/dx at the cell centroid (cell.tcc:33-65), once per cell of a general mesh (CentroidGrad)
-  h->dndx_c.resize((size_t)ncells * nv * dim);
-  for (int64_t c = 0; c < ncells; ++c) {
-    for (int i = 0; i < nv; ++i) {
-      const int64_t n = cell_nodes[c * nv + i];
-      for (int d = 0; d < dim; ++d) X[i * dim + d] = coords[n * dim + d];
-    }
-    double xi0[3] = {0., 0., 0.};
-    if (dim == 2)
-      dn_dx<2>(xi0, X.data(), &h->dndx_c[(size_t)c * nv * dim]);
-    else
-      dn_dx<3>(xi0, X.data(), &h->dndx_c[(size_t)c * nv * dim]);
   }
   std::vector<std::vector<int32_t>> node_cells(nnodes);
   for (int64_t c = 0; c < ncells; ++c)

@@ -149,7 +149,7 @@ struct DevState {
   int32_t* nc_off = nullptr;     // [nn + 1]
   int32_t* nc_cell = nullptr;
   int8_t* nc_slot = nullptr;
-  double* dndx_c = nullptr;      // general meshes: [ncells][NV][DIM] dN/dx at the cell centroid
+  double* dndx_c = nullptr;      // [ncells][NV][DIM] dN/dx at the cell centroid
 
   // per-step counting sort of particles by cell and the cell-slot partial
   // sums of P2G (mass, momentum, external force, internal force per slot)
@@ -183,7 +183,7 @@ struct DevState {
   float* svf = nullptr;           // [SVF_N][np]
   float* nfv = nullptr;           // [nn][nfv_stride(DIM)] nodal velocity, acceleration
   float* partials_f = nullptr;    // [ncells][NV][1 + 3 DIM]
-  float* dndx_cf = nullptr;       // general meshes: [ncells][NV][DIM]
+  float* dndx_cf = nullptr;       // [ncells][NV][DIM]
   const MaterialT<float>* mats_f = nullptr;
 
   int remove_lost = 0;            // locate_particles false: unlocatable particles are removed
