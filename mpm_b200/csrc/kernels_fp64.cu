@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(T, (tile_min_blocks<BOX, AFF, T>()))
       for (int d = 0; d < DIM; ++d) rows[RW::XI + d][t] = xi[d];
       if constexpr (MM && AFF) {
         double Mv[DIM * DIM];
-        mapping_velocity_matrix<DIM, AFF, BOX>(s, p, pc, x, xi, Mv);
+        mapping_velocity_matrix<DIM, AFF, false>(s, p, pc, x, xi, Mv);  // the reference's sums and inverse
 #pragma unroll
         for (int d = 0; d < DIM; ++d) rows[RW::XP + d][t] = x[d];
 #pragma unroll

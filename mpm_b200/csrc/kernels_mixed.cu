@@ -19,6 +19,7 @@
 //     P = V / V0 - 1) so that FP32 keeps the 1e-9 per-step increments.
 // Same step structure as the FP64 path (kernels_fp64.cu): counting sort,
 // per-cell P2G, node gather and update, G2P + stress + locate.
+#define MPM_MC_RECIPROCALS  // see mpm_math.cuh
 #include <cuda_runtime.h>
 
 #include <cstdint>

@@ -138,9 +138,11 @@ MPM_HD Dual pow(const Dual& a, double e) {
 MPM_HD Dual pow(const Dual& a, const Dual& e) { return pow(a, e.v); }  // constant exponents only
 MPM_HD Dual fabs(const Dual& a) { return a.v < 0.0 ? -a : a; }
 MPM_HD bool isfinite(const Dual& a) { return a.v - a.v == 0.0; }
-MPM_HD Dual rsqrt_of(const Dual& a) {
-  const double s = rsqrt_of(a.v);
-  return chain(a, s, -0.5 * s * s * s);
+MPM_HD void sin_cos(const Dual& x, Dual* sn, Dual* cs) {
+  double s, c;
+  sin_cos(x.v, &s, &c);
+  *sn = chain(x, s, c);
+  *cs = chain(x, c, -s);
 }
 MPM_HD double value(const Dual& a) { return a.v; }
 
@@ -154,22 +156,6 @@ MPM_HD double value(const Dual& a) { return a.v; }
 template <>
 MPM_HD Dual lode_corner<Dual>(const Dual& x, double dist_to_corner) {
   return dist_to_corner < MPM_LODE_CORNER_TOL ? Dual(x.v) : x;
-}
-
-// d theta / dv of theta = acos(v) / 3, zero in the corners
-MPM_HD void lode_trig(const Dual& v, Dual* sn, Dual* cs) {
-  double s, c;
-  lode_trig(v.v, &s, &c);
-  const double q = 1.0 - v.v * v.v;
-  const double dt = q < MPM_LODE_CORNER_TOL ? 0.0 : (-1.0 / 3.0) / ::sqrt(q);
-  *sn = chain(v, s, c * dt);
-  *cs = chain(v, c, -s * dt);
-}
-MPM_HD Dual lode_theta(const Dual& sn, const Dual& cs) {
-  Dual r(lode_theta(sn.v, cs.v));
-#pragma unroll
-  for (int k = 0; k < NT; ++k) r.d[k] = cs.v * sn.d[k] - sn.v * cs.d[k];
-  return r;
 }
 
 template <>

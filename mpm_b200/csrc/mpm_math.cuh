@@ -441,11 +441,19 @@ template <typename R>
 MPM_HD R sq(R x) {
   return x * x;
 }
+#ifdef MPM_MC_RECIPROCALS
 template <typename R>
 MPM_HD R mu_j2(const R* s) {
   return (sq(s[0] - s[1]) + sq(s[1] - s[2]) + sq(s[0] - s[2])) * (R(1) / R(6)) + sq(s[3]) + sq(s[4]) +
          sq(s[5]);
 }
+#else
+template <typename R>
+MPM_HD R mu_j2(const R* s) {
+  return (sq(s[0] - s[1]) + sq(s[1] - s[2]) + sq(s[0] - s[2])) / R(6) + sq(s[3]) + sq(s[4]) +
+         sq(s[5]);
+}
+#endif
 template <typename R>
 MPM_HD R mu_j3(const R* s) {
   const R p = mu_p(s);
@@ -472,6 +480,16 @@ MPM_HD T lode_corner(const T& x, double /*dist_to_corner*/) {
 MPM_HD double value(double x) { return x; }
 MPM_HD float value(float x) { return x; }
 
+enum { MC_ELASTIC = 0, MC_SHEAR = 1, MC_TENSILE = 2, MC_SEPARATED = 3 };
+
+// The invariants, yield state and flow directions come in two forms of the same
+// formulas.  As written by the reference, operation by operation, for the FP64
+// path and its derivatives: a cohesive column amplifies one rounding near an apex
+// to 1e-6 of the stress within a hundred steps, so any other order of operations
+// parts from the reference's run there.  With reciprocals and the triple-angle
+// equation (MPM_MC_RECIPROCALS) for the mixed path, whose FP32 state sets its
+// error: returns of 0.8M flowing points 205 -> 123 us.
+#ifdef MPM_MC_RECIPROCALS
 // 1 / sqrt(x)
 MPM_HD float rsqrt_of(float x) {
 #ifdef __CUDA_ARCH__
@@ -616,7 +634,6 @@ MPM_HD R mc_lode_angle(const LodeTrig<R>& lt) {
   return R(lode_theta(lt.hs, lt.hc));
 }
 
-enum { MC_ELASTIC = 0, MC_SHEAR = 1, MC_TENSILE = 2, MC_SEPARATED = 3 };
 
 // mohr_coulomb.tcc:139-191
 template <typename R>
@@ -649,8 +666,8 @@ MPM_HD int mc_yield_state(R* yf, const R* sv, const LodeTrig<R>& lt, const Frict
 // divided by are taken as reciprocal ones: 4 of them for a shear point where
 // the formulas as written have 25.
 // With lode_trig: the plastic returns of a flowing column (0.8M points) 205 ->
-// 123 us mixed, of 256k points in FP64 60 -> 43 us; within 1e-13 of the formulas
-// as written on random states, the same number of corrections.
+// 123 us; within 1e-13 of the formulas as written on random states, the same
+// number of corrections.
 template <typename R>
 MPM_HD void mc_df_dp(const MaterialT<R>& m, int yield_type, const R* sv, const LodeTrig<R>& lt,
                      const FrictionTrig<R>& ft, R pdstrain, const R* s, R* df, R* dp, R* dp_dq,
@@ -789,6 +806,261 @@ MPM_HD void mc_df_dp(const MaterialT<R>& m, int yield_type, const R* sv, const L
     *softening = R(-1) * ((df_dphi * dphi_dpstrain) + (df_dc * dc_dpstrain)) * (*dp_dq);
   }
 }
+
+#else  // as written
+// sin and cos of an FP64 angle in one evaluation
+MPM_HD void sin_cos(double x, double* sn, double* cs) {
+#ifdef __CUDA_ARCH__
+  sincos(x, sn, cs);
+#else
+  *sn = std::sin(x);
+  *cs = std::cos(x);
+#endif
+}
+
+// Trigonometric values of the Lode angle theta of one invariant evaluation:
+// cos, sin of theta, theta + pi/3 and theta - 4 pi/3 all follow from one
+// sin/cos evaluation of theta by the angle-addition formulas.
+template <typename R>
+struct LodeTrig {
+  R ct, st;    // cos theta, sin theta
+  R sp3, cp3;  // sin (theta + pi/3), cos (theta + pi/3)
+  R cm43;      // cos (theta - 4 pi/3)
+  R theta;
+};
+// Friction and dilation angle functions of one return (fixed during a
+// return: softening moves phi and psi only before the predictor).
+template <typename R>
+struct FrictionTrig {
+  R sphi, cphi, tphi, tpsi;
+};
+
+template <typename R>
+MPM_HD FrictionTrig<R> friction_trig(const MaterialT<R>& m, const R* sv) {
+  FrictionTrig<R> t;
+  if (sv[SV_PHI] == m.phi_peak && sv[SV_PSI] == m.psi_peak) {
+    t.sphi = m.sin_phi;
+    t.cphi = m.cos_phi;
+    t.tphi = m.tan_phi;
+    t.tpsi = m.tan_psi;
+  } else {
+    t.sphi = sin(sv[SV_PHI]);
+    t.cphi = cos(sv[SV_PHI]);
+    t.tphi = tan(sv[SV_PHI]);
+    t.tpsi = tan(sv[SV_PSI]);
+  }
+  return t;
+}
+
+// mohr_coulomb.tcc:124-134 with lode_angle (material_utility.tcc:65-81).
+// Evaluated in FP64 for every working precision R: the Lode angle is acos of
+// a ratio that reaches +-1 on triaxial stress paths (a geostatic K0 state is
+// one), where acos turns a rounding error e of the ratio into an angle error
+// of about sqrt(2e) -- 5e-4 rad from FP32 rounding, which moves the returned
+// stress by 1e-4 of its magnitude.
+template <typename R>
+MPM_HD void mc_invariants(const R* s, R* sv, LodeTrig<R>& lt) {
+  using H = typename HighPrecision<R>::T;
+  const H d[6] = {H(s[0]), H(s[1]), H(s[2]), H(s[3]), H(s[4]), H(s[5])};
+  const H j2 = mu_j2(d);
+  const H j3 = mu_j3(d);
+  sv[SV_EPS] = R(mu_p(d) * sqrt(3.0));
+  H v = H(0.0);
+  if (fabs(j2) > kDblEps) v = (3.0 * sqrt(3.0) / 2.0) * (j3 / (j2 * sqrt(j2)));
+  if (v > 1.0) v = H(1.0);
+  if (v < -1.0) v = H(-1.0);
+  const H theta = lode_corner((1.0 / 3.0) * acos(v), value(1.0 - v * v));
+  lt.theta = R(theta);
+  sv[SV_RHO] = R(sqrt(2.0 * j2));
+  H sn, cs;
+  sin_cos(theta, &sn, &cs);
+  const double h = 0.5, r3 = 0.86602540378443864676;  // cos, sin of pi/3
+  lt.ct = R(cs);
+  lt.st = R(sn);
+  lt.sp3 = R(sn * h + cs * r3);
+  lt.cp3 = R(cs * h - sn * r3);
+  lt.cm43 = R(-(cs * h) - sn * r3);
+}
+
+template <typename R>
+MPM_HD R mc_lode_angle(const LodeTrig<R>& lt) {
+  return lt.theta;
+}
+
+
+// mohr_coulomb.tcc:139-191
+template <typename R>
+MPM_HD int mc_yield_state(R* yf, const R* sv, const LodeTrig<R>& lt, const FrictionTrig<R>& ft) {
+  const R Tolerance = R(-1E-1);
+  const R epsilon = sv[SV_EPS], rho = sv[SV_RHO];
+  const R cohesion = sv[SV_COH], tension_cutoff = sv[SV_TC];
+  yf[0] = sqrt(R(2) / R(3)) * lt.ct * rho + epsilon / sqrt(R(3)) - tension_cutoff;
+  yf[1] = sqrt(R(1.5)) * rho * ((lt.sp3 / (sqrt(R(3)) * ft.cphi)) + (lt.cp3 * ft.tphi / R(3))) +
+          (epsilon / sqrt(R(3))) * ft.tphi - cohesion;
+  int yield_type = MC_ELASTIC;
+  if (yf[0] > Tolerance && yf[1] > Tolerance) {
+    const R n_phi = (R(1) + ft.sphi) / (R(1) - ft.sphi);
+    const R sigma_p = tension_cutoff * n_phi - R(2) * cohesion * sqrt(n_phi);
+    const R alpha_p = sqrt(R(1) + n_phi * n_phi) + n_phi;
+    const R h = yf[0] + alpha_p * (sqrt(R(2) / R(3)) * lt.cm43 * rho + epsilon / sqrt(R(3)) - sigma_p);
+    yield_type = (h > dbl_eps<R>()) ? MC_TENSILE : MC_SHEAR;
+  }
+  if (yf[0] < Tolerance && yf[1] > Tolerance) yield_type = MC_SHEAR;
+  if (yf[0] > Tolerance && yf[1] < Tolerance) yield_type = MC_TENSILE;
+  return yield_type;
+}
+
+// mohr_coulomb.tcc:195-344 (dF/dsigma, dP/dsigma, dP/dq, softening).  pdstrain
+// is passed separately (it is kept in FP64 on every path).
+template <typename R>
+MPM_HD void mc_df_dp(const MaterialT<R>& m, int yield_type, const R* sv, const LodeTrig<R>& lt,
+                     const FrictionTrig<R>& ft, R pdstrain, const R* s, R* df, R* dp, R* dp_dq,
+                     R* softening) {
+  const R eps = dbl_eps<R>();
+  const R rho = sv[SV_RHO];
+  const R phi = sv[SV_PHI], tension_cutoff = sv[SV_TC];
+  const R ct = lt.ct, st = lt.st;
+  R df_depsilon, df_drho, df_dtheta;
+  if (yield_type == MC_TENSILE) {
+    df_depsilon = R(1) / sqrt(R(3));
+    df_drho = sqrt(R(2) / R(3)) * ct;
+    df_dtheta = -sqrt(R(2) / R(3)) * rho * st;
+  } else {
+    df_depsilon = ft.tphi / sqrt(R(3));
+    df_drho = sqrt(R(1.5)) * ((lt.sp3 / (sqrt(R(3)) * ft.cphi)) + (lt.cp3 * ft.tphi / R(3)));
+    df_dtheta = sqrt(R(1.5)) * rho * ((lt.cp3 / (sqrt(R(3)) * ft.cphi)) - (lt.sp3 * ft.tphi / R(3)));
+  }
+  // dEpsilon/dsigma = dp/dsigma * sqrt(3); dRho/dsigma = dq/dsigma * sqrt(2/3)
+  const R deps_ds = R(1) / R(3) * sqrt(R(3));
+  const R j2 = mu_j2(s);
+  const R q = sqrt(R(3) * j2);
+  const R pm = mu_p(s);
+  const R dev[6] = {s[0] - pm, s[1] - pm, s[2] - pm, s[3], s[4], s[5]};
+  R drho_ds[6] = {R(0), R(0), R(0), R(0), R(0), R(0)};
+  if (fabs(q) > eps) {
+    drho_ds[0] = R(3) / (R(2) * q) * dev[0];
+    drho_ds[1] = R(3) / (R(2) * q) * dev[1];
+    drho_ds[2] = R(3) / (R(2) * q) * dev[2];
+    drho_ds[3] = R(3) / q * dev[3];
+    drho_ds[4] = R(3) / q * dev[4];
+    drho_ds[5] = R(3) / q * dev[5];
+  }
+#pragma unroll
+  for (int i = 0; i < 6; ++i) drho_ds[i] *= sqrt(R(2) / R(3));
+  // dtheta/dsigma (material_utility.tcc:166-200), in FP64 for every R for
+  // the reason given at mc_invariants (1 - r^2 vanishes on triaxial paths)
+  R dtheta_ds[6];
+  {
+    using H = typename HighPrecision<R>::T;
+    const H sd[6] = {H(s[0]), H(s[1]), H(s[2]), H(s[3]), H(s[4]), H(s[5])};
+    const H j2d = mu_j2(sd);
+    const H pmd = mu_p(sd);
+    const H dv[6] = {sd[0] - pmd, sd[1] - pmd, sd[2] - pmd, sd[3], sd[4], sd[5]};
+    const H j3 = mu_j3(sd);
+    const H dj2[6] = {dv[0], dv[1], dv[2], dv[3] * 2.0, dv[4] * 2.0, dv[5] * 2.0};
+    const H dev1[3] = {dv[0], dv[3], dv[5]};
+    const H dev2[3] = {dv[3], dv[1], dv[4]};
+    const H dev3[3] = {dv[5], dv[4], dv[2]};
+    auto dot3 = [](const H* a, const H* b) { return (a[0] * b[0] + a[1] * b[1]) + a[2] * b[2]; };
+    const H dj3[6] = {dot3(dev1, dev1) - (2.0 / 3.0) * j2d,
+                      dot3(dev2, dev2) - (2.0 / 3.0) * j2d,
+                      dot3(dev3, dev3) - (2.0 / 3.0) * j2d,
+                      2.0 * dot3(dev1, dev2),
+                      2.0 * dot3(dev2, dev3),
+                      2.0 * dot3(dev1, dev3)};
+    H dr_dj2 = -9.0 / 4.0 * sqrt(3.0) * j3;
+    H dr_dj3 = H(3.0 / 2.0 * sqrt(3.0));
+    H dtheta_dr = H(-1.0 / 3.0);
+    if (fabs(j2d) > kDblEps) {
+      // j2^-1.5 and j2^-2.5 from one square root
+      const H p15 = 1.0 / (j2d * sqrt(j2d));
+      const H r = j3 / 2.0 * (3.0 * sqrt(3.0)) * p15;
+      dr_dj2 *= p15 / j2d;
+      dr_dj3 *= p15;
+      const H factor = lode_corner((fabs(1.0 - r * r) < kDblEps) ? H(kDblEps) : fabs(1.0 - r * r),
+                                   value(fabs(1.0 - r * r)));
+      dtheta_dr = -1.0 / (3.0 * sqrt(factor));
+    }
+#pragma unroll
+    for (int i = 0; i < 6; ++i) dtheta_ds[i] = R(dtheta_dr * ((dr_dj2 * dj2[i]) + (dr_dj3 * dj3[i])));
+  }
+#pragma unroll
+  for (int i = 0; i < 6; ++i)
+    df[i] = ((df_depsilon * (i < 3 ? deps_ds : R(0))) + (df_drho * drho_ds[i])) +
+            (df_dtheta * dtheta_ds[i]);
+  if (yield_type == MC_TENSILE) {
+    const R et_value = R(0.6);
+    const R xit = R(0.1);
+    R sqpart = R(4) * (R(1) - et_value * et_value) * ct * ct + R(5) * et_value * et_value -
+               R(4) * et_value;
+    if (sqpart < eps) sqpart = R(1.E-5);
+    R rt_den = R(2) * (R(1) - et_value * et_value) * ct + (R(2) * et_value - R(1)) * sqrt(sqpart);
+    const R rt_num = R(4) * (R(1) - et_value * et_value) * ct * ct +
+                     (R(2) * et_value - R(1)) * (R(2) * et_value - R(1));
+    if (fabs(rt_den) < eps) rt_den = R(1.E-5);
+    const R rt = rt_num / (R(3) * rt_den);
+    const R den = check_low(
+        sqrt(xit * xit * tension_cutoff * tension_cutoff + R(1.5) * rt * rt * rho * rho));
+    const R dp_drt = R(1.5) * rho * rho * rt / den;
+    const R dp_drho = R(1.5) * rho * rt * rt / den;
+    const R dp_depsilon = R(1) / sqrt(R(3));
+    const R drtden_dtheta =
+        R(-2) * (R(1) - et_value * et_value) * st -
+        (R(2) * et_value - R(1)) * R(4) * (R(1) - et_value * et_value) * ct * st /
+            sqrt(R(4) * (R(1) - et_value * et_value) * ct * ct + R(5) * et_value * et_value -
+                 R(4) * et_value);
+    const R drtnum_dtheta = R(-8) * (R(1) - et_value * et_value) * ct * st;
+    const R drt_dtheta =
+        (drtnum_dtheta * rt_den - drtden_dtheta * rt_num) / (R(3) * rt_den * rt_den);
+#pragma unroll
+    for (int i = 0; i < 6; ++i)
+      dp[i] = ((dp_depsilon * (i < 3 ? deps_ds : R(0))) + (dp_drho * drho_ds[i])) +
+              (dp_drt * drt_dtheta * dtheta_ds[i]);
+    *dp_dq = dp_drho * sqrt(R(2) / R(3));
+  } else {
+    const R sphi = ft.sphi, cphi = ft.cphi;
+    const R r_mc = (R(3) - sphi) / (R(6) * cphi);
+    R e_val = (R(3) - sphi) / (R(3) + sphi);
+    if (e_val <= R(0.5)) e_val = R(0.5) + R(1.E-10);
+    if (e_val > R(1)) e_val = R(1);
+    R sqpart = (R(4) * (R(1) - e_val * e_val) * sq(ct)) + (R(5) * e_val * e_val) - (R(4) * e_val);
+    if (sqpart < eps) sqpart = R(1.E-5);
+    R mm = (R(2) * (R(1) - e_val * e_val) * ct) + ((R(2) * e_val - R(1)) * sqrt(sqpart));
+    if (fabs(mm) < eps) mm = R(1.E-5);
+    const R l = (R(4) * (R(1) - e_val * e_val) * sq(ct)) + sq(R(2) * e_val - R(1));
+    const R r_mw = (l / mm) * r_mc;
+    const R xi = R(0.1);
+    R omega = sq(xi * m.c_peak * ft.tpsi) + sq(r_mw * sqrt(R(1.5)) * rho);
+    if (omega < eps) omega = R(1.E-5);
+    const R dl_dtheta = R(-8) * (R(1) - e_val * e_val) * ct * st;
+    const R dm_dtheta = (R(-2) * (R(1) - e_val * e_val) * st) +
+                        (R(0.5) * (R(2) * e_val - R(1)) * dl_dtheta) / sqrt(sqpart);
+    const R drmw_dtheta = ((mm * dl_dtheta) - (l * dm_dtheta)) / (mm * mm);
+    const R dp_depsilon = ft.tpsi / sqrt(R(3));
+    const R dp_drho = R(3) * rho * r_mw * r_mw / (R(2) * sqrt(omega));
+    const R dp_dtheta = (R(3) * rho * rho * r_mw * r_mc * drmw_dtheta) / (R(2) * sqrt(omega));
+#pragma unroll
+    for (int i = 0; i < 6; ++i)
+      dp[i] = ((dp_depsilon * (i < 3 ? deps_ds : R(0))) + (dp_drho * drho_ds[i])) +
+              (dp_dtheta * dtheta_ds[i]);
+    *dp_dq = dp_drho * sqrt(R(2) / R(3));
+  }
+  *softening = R(0);
+  if (m.softening && pdstrain > m.pd_peak && pdstrain < m.pd_res) {
+    const R dphi_dpstrain = (m.phi_res - m.phi_peak) / (m.pd_res - m.pd_peak);
+    const R dc_dpstrain = (m.c_res - m.c_peak) / (m.pd_res - m.pd_peak);
+    const R df_dphi =
+        sqrt(R(1.5)) * rho *
+            ((ft.sphi * lt.sp3 / (sqrt(R(3)) * ft.cphi * ft.cphi)) +
+             (lt.cp3 / (R(3) * ft.cphi * ft.cphi))) +
+        (mu_p(s) / (ft.cphi * ft.cphi));
+    const R df_dc = R(-1);
+    *softening = R(-1) * ((df_dphi * dphi_dpstrain) + (df_dc * dc_dpstrain)) * (*dp_dq);
+  }
+  (void)phi;
+}
+
+#endif
 
 // Out-of-line copies of the three heavy pieces of the return map, for the
 // full (non-deferred) update: it evaluates each at up to four places (trial
