@@ -1164,13 +1164,13 @@ void step_impl(const DevState& s, const StepArgs& a, cudaStream_t st, Profiler& 
   };
   if (a.scheme == 1 && a.phase == 2) goto usl_second_half;
   if (a.returns_first) {
-    fork_side(a, st);
+    check_cuda(fork_side(a, st), "returns beside the sort: fork");
     returns_fp64<DIM>(s, a, a.side, pr);
   }
   pr.begin(K_SORT, st, sort_kernels(s));
   counting_sort_impl(s, st, 1);
   pr.end(K_SORT, st);
-  if (a.returns_first) join_side(a, st);
+  if (a.returns_first) check_cuda(join_side(a, st), "returns beside the sort: join");
   if (a.scheme == 2) {  // MUSL (mpm_scheme_musl.tcc)
     pr.begin(K_P2G, st);
     p2g(std::integral_constant<int, 2>{});

@@ -1602,13 +1602,13 @@ void step_mixed(const DevState& s, const StepArgs& a, cudaStream_t st, Profiler&
   };
   if (a.scheme == 1 && a.phase == 2) goto usl_second_half;
   if (a.returns_first) {
-    fork_side(a, st);
+    check_cuda(fork_side(a, st), "returns beside the sort: fork");
     returns_mixed<DIM>(s, a, a.side, pr);
   }
   pr.begin(K_SORT, st, sort_kernels(s));
   counting_sort(s, st, 1);
   pr.end(K_SORT, st);
-  if (a.returns_first) join_side(a, st);
+  if (a.returns_first) check_cuda(join_side(a, st), "returns beside the sort: join");
   if (a.scheme == 2) {  // MUSL (mpm_scheme_musl.tcc:20-35)
     pr.begin(K_P2G, st);
     p2g(std::integral_constant<int, 2>{});

@@ -198,6 +198,8 @@ void parallel_for(int64_t n, F f) {
 
 namespace mpm_b200 {
 
+void check_cuda(cudaError_t e, const char* what) { ck(e, what); }
+
 const char* kernel_name(int kid) {
   static const char* names[K_NKERNELS] = {"sort",  "p2g",   "nodes_velocity", "stress",
                                           "p2g_forces", "nodes_acceleration", "g2p",
@@ -1908,20 +1910,28 @@ static int run_steps(mpm_gpu_t h, int64_t nsteps, double* elapsed_ms) {
       h->graph = nullptr;
       const int64_t l0 = h->prof.launches;
       cudaGraph_t g = nullptr;
-      bool ok = cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
-      if (ok) {
-        launch();
-        ok = cudaStreamEndCapture(h->stream, &g) == cudaSuccess && g != nullptr;
-        ok = ok && cudaGraphInstantiate(&h->graph, g, 0) == cudaSuccess;
-        if (g) cudaGraphDestroy(g);
+      std::string why;
+      try {
+        ck(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal), "begin capture");
+        try {
+          launch();
+        } catch (const CudaError& e) {
+          why = e.what();
+        }
+        ck(cudaStreamEndCapture(h->stream, &g), "end capture");  // also of a capture that a launch broke
+        if (why.empty()) ck(cudaGraphInstantiate(&h->graph, g, 0), "instantiate");
+      } catch (const CudaError& e) {
+        if (why.empty()) why = e.what();
       }
-      if (ok) {
+      if (g) cudaGraphDestroy(g);
+      if (why.empty()) {
         h->graph_state = h->ds;
         h->graph_args = a;
         h->graph_launches = h->prof.launches - l0;
         ck(cudaGraphLaunch(h->graph, h->stream), "cudaGraphLaunch");
       } else {  // capture not possible here: launch eagerly from now on
         cudaGetLastError();
+        h->err = "the steps are launched without a graph: " + why;
         if (h->graph) cudaGraphExecDestroy(h->graph);
         h->graph = nullptr;
         h->graph_ok = false;

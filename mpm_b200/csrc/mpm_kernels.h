@@ -134,15 +134,18 @@ cudaError_t launch_steps_persistent_mixed(int dim, const DevState& s, const Step
 // (words: it also resets the length of the list of lost particles; that of the
 // plastic points is reset by the node update, see StepArgs::returns_first)
 void counting_sort(const DevState& s, cudaStream_t st, int words = 0);
-// the fork and join of StepArgs::returns_first
-inline void fork_side(const StepArgs& a, cudaStream_t st) {
-  cudaEventRecord(a.fork, st);
-  cudaStreamWaitEvent(a.side, a.fork, 0);
+// The fork and join of StepArgs::returns_first.  Their codes are to be checked:
+// without the join P2G would run beside the returns.
+[[nodiscard]] inline cudaError_t fork_side(const StepArgs& a, cudaStream_t st) {
+  const cudaError_t e = cudaEventRecord(a.fork, st);
+  return e != cudaSuccess ? e : cudaStreamWaitEvent(a.side, a.fork, 0);
 }
-inline void join_side(const StepArgs& a, cudaStream_t st) {
-  cudaEventRecord(a.join, a.side);
-  cudaStreamWaitEvent(st, a.join, 0);
+[[nodiscard]] inline cudaError_t join_side(const StepArgs& a, cudaStream_t st) {
+  const cudaError_t e = cudaEventRecord(a.join, a.side);
+  return e != cudaSuccess ? e : cudaStreamWaitEvent(st, a.join, 0);
 }
+// throws, with the call's name, unless e is cudaSuccess
+void check_cuda(cudaError_t e, const char* what);
 void launch_locate_fallback(int dim, const DevState& s, int remove_lost, cudaStream_t st);
 // PODParticle records (pod_particle.h:12-62): 74 fields, caller's layout
 constexpr int POD_NFIELDS = 74;
