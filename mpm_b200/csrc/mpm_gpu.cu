@@ -390,6 +390,7 @@ struct mpm_gpu_solver {
   // a step's plastic returns beside the next one's sort (StepArgs::returns_first)
   cudaStream_t side = nullptr;
   cudaEvent_t fork = nullptr, join = nullptr;
+  bool returns_launched = false;  // some step has launched its returns outside a capture
 
   // launch shape of the value steps (mpm_gpu_set_launch_shape, mpm_gpu_autotune);
   // zeros are the built-in defaults
@@ -1880,8 +1881,11 @@ static int run_steps(mpm_gpu_t h, int64_t nsteps, double* elapsed_ms) {
   }
   // A step whose device state and arguments match the captured one replays the
   // captured CUDA graph (one graph launch instead of the step's kernel
-  // launches).  The first step of a call runs eagerly (it sets the kernels'
-  // shared-memory attributes outside any capture); profiling runs eagerly.
+  // launches).  Every kernel of a step is launched eagerly before a capture of
+  // it (the first launch sets shared-memory attributes and loads the kernel):
+  // the first step of a call, and of a handle's first call that defers its
+  // returns also the second, which is the first to make any.  Profiling runs
+  // eagerly.
   bool eager_done = false;
   // Each step's plastic returns run beside the next step's sort; the call's last
   // ones after its last step.
@@ -1901,7 +1905,7 @@ static int run_steps(mpm_gpu_t h, int64_t nsteps, double* elapsed_ms) {
     if (h->cfg.gravity_ramping_time > 0.0)
       gm = std::min(1.0, static_cast<double>(h->step) * h->cfg.dt / h->cfg.gravity_ramping_time);
     for (int d = 0; d < 3; ++d) a.g[d] = d < h->dim ? gm * h->cfg.gravity[d] : 0.;
-    const bool graphable = h->graph_ok && !h->prof.enabled && eager_done;
+    const bool graphable = h->graph_ok && !h->prof.enabled && eager_done && (!beside || h->returns_launched);
     if (graphable && h->graph && same_step(h->graph_state, h->ds, h->graph_args, a)) {
       ck(cudaGraphLaunch(h->graph, h->stream), "cudaGraphLaunch");
       h->prof.launches += h->graph_launches;
@@ -1941,6 +1945,7 @@ static int run_steps(mpm_gpu_t h, int64_t nsteps, double* elapsed_ms) {
     } else {
       launch();
       eager_done = true;
+      h->returns_launched = h->returns_launched || !beside || a.returns_first;
     }
     ck(cudaGetLastError(), "kernel launch");
     ++h->step;
@@ -1951,6 +1956,7 @@ static int run_steps(mpm_gpu_t h, int64_t nsteps, double* elapsed_ms) {
     else
       launch_returns_fp64(h->dim, h->ds, a, h->stream, h->prof);
     ck(cudaGetLastError(), "kernel launch");
+    h->returns_launched = true;
   }
   if (elapsed_ms) ck(cudaEventRecord(e1, h->stream), "cudaEventRecord");
   unsigned words[2] = {0, 0};
@@ -2087,9 +2093,9 @@ int mpm_gpu_autotune(mpm_gpu_t h, int64_t steps, char* report, size_t report_len
         *field[f] = cand[f][k];
         copy(false);
         h->step = step0;
-        // two untimed steps (an eager one, then the graph capture), then the
+        // three untimed steps (eager ones, then the graph capture), then the
         // timed ones (an eager step, then graph replays)
-        rc = run_steps(h, 2, nullptr);
+        rc = run_steps(h, 3, nullptr);
         double ms = 0.;
         if (rc == MPM_OK) rc = run_steps(h, steps, &ms);
         js += std::string(k ? ", " : "") + "\"" + std::to_string(cand[f][k]) + "\": " +
