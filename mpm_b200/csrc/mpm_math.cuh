@@ -441,19 +441,6 @@ template <typename R>
 MPM_HD R sq(R x) {
   return x * x;
 }
-#ifdef MPM_MC_RECIPROCALS
-template <typename R>
-MPM_HD R mu_j2(const R* s) {
-  return (sq(s[0] - s[1]) + sq(s[1] - s[2]) + sq(s[0] - s[2])) * (R(1) / R(6)) + sq(s[3]) + sq(s[4]) +
-         sq(s[5]);
-}
-#else
-template <typename R>
-MPM_HD R mu_j2(const R* s) {
-  return (sq(s[0] - s[1]) + sq(s[1] - s[2]) + sq(s[0] - s[2])) / R(6) + sq(s[3]) + sq(s[4]) +
-         sq(s[5]);
-}
-#endif
 template <typename R>
 MPM_HD R mu_j3(const R* s) {
   const R p = mu_p(s);
@@ -480,6 +467,16 @@ MPM_HD T lode_corner(const T& x, double /*dist_to_corner*/) {
 MPM_HD double value(double x) { return x; }
 MPM_HD float value(float x) { return x; }
 
+// sin and cos of an FP64 angle in one evaluation
+MPM_HD void sin_cos(double x, double* sn, double* cs) {
+#ifdef __CUDA_ARCH__
+  sincos(x, sn, cs);
+#else
+  *sn = std::sin(x);
+  *cs = std::cos(x);
+#endif
+}
+
 enum { MC_ELASTIC = 0, MC_SHEAR = 1, MC_TENSILE = 2, MC_SEPARATED = 3 };
 
 // The invariants, yield state and flow directions come in two forms of the same
@@ -489,7 +486,23 @@ enum { MC_ELASTIC = 0, MC_SHEAR = 1, MC_TENSILE = 2, MC_SEPARATED = 3 };
 // parts from the reference's run there.  With reciprocals and the triple-angle
 // equation (MPM_MC_RECIPROCALS) for the mixed path, whose FP32 state sets its
 // error: returns of 0.8M flowing points 205 -> 123 us.
+//
+// A unit has one form; all that depends on it, here and in mpm_return.cuh, is in a
+// namespace of the form's name, so that units of both forms can be linked into one
+// program, on the host and as relocatable device code.
 #ifdef MPM_MC_RECIPROCALS
+#define MPM_MC_FORM mc_reciprocal
+#else
+#define MPM_MC_FORM mc_as_written
+#endif
+inline namespace MPM_MC_FORM {
+
+#ifdef MPM_MC_RECIPROCALS
+template <typename R>
+MPM_HD R mu_j2(const R* s) {
+  return (sq(s[0] - s[1]) + sq(s[1] - s[2]) + sq(s[0] - s[2])) * (R(1) / R(6)) + sq(s[3]) + sq(s[4]) +
+         sq(s[5]);
+}
 // 1 / sqrt(x)
 MPM_HD float rsqrt_of(float x) {
 #ifdef __CUDA_ARCH__
@@ -808,16 +821,11 @@ MPM_HD void mc_df_dp(const MaterialT<R>& m, int yield_type, const R* sv, const L
 }
 
 #else  // as written
-// sin and cos of an FP64 angle in one evaluation
-MPM_HD void sin_cos(double x, double* sn, double* cs) {
-#ifdef __CUDA_ARCH__
-  sincos(x, sn, cs);
-#else
-  *sn = std::sin(x);
-  *cs = std::cos(x);
-#endif
+template <typename R>
+MPM_HD R mu_j2(const R* s) {
+  return (sq(s[0] - s[1]) + sq(s[1] - s[2]) + sq(s[0] - s[2])) / R(6) + sq(s[3]) + sq(s[4]) +
+         sq(s[5]);
 }
-
 // Trigonometric values of the Lode angle theta of one invariant evaluation:
 // cos, sin of theta, theta + pi/3 and theta - 4 pi/3 all follow from one
 // sin/cos evaluation of theta by the angle-addition formulas.
@@ -1060,7 +1068,7 @@ MPM_HD void mc_df_dp(const MaterialT<R>& m, int yield_type, const R* sv, const L
   (void)phi;
 }
 
-#endif
+#endif  // MPM_MC_RECIPROCALS
 
 // Out-of-line copies of the three heavy pieces of the return map, for the
 // full (non-deferred) update: it evaluates each at up to four places (trial
@@ -1260,6 +1268,8 @@ MPM_HD void material_compute_stress(const MaterialParams& m, const double* stres
   }
   mc_compute_stress<double, double>(m, stress, dstrain, density, sv, sv[SV_PD], out, corrections);
 }
+
+}  // namespace MPM_MC_FORM
 
 // ---------------------------------------------------------------- node update
 struct NodeBC {

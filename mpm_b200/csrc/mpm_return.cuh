@@ -19,6 +19,7 @@
 #include "mpm_math.cuh"
 
 namespace mpm_b200 {
+inline namespace MPM_MC_FORM {
 
 enum { MR_OLD = 0, MR_TRIAL, MR_LOOP, MR_FINAL };
 
@@ -176,4 +177,5 @@ __device__ __forceinline__ void mc_return(const MaterialT<R>& m, const R* stress
   *corrections = q.itr;
 }
 
+}  // namespace MPM_MC_FORM
 }  // namespace mpm_b200
