@@ -727,16 +727,12 @@ void make_tangent_materials(const MaterialParams* mats, int nmats, const Tangent
       r.cos_phi = cos(r.phi_peak);
       r.tan_phi = tan(r.phi_peak);
       r.tan_psi = tan(r.psi_peak);
-      friction_quotients(r.sin_phi, r.cos_phi, r.ic_phi, r.e_phi, r.n_phi);
       // the values must be the FP64 material's
       r.tc_init.v = m.tc_init;
       r.sin_phi.v = m.sin_phi;
       r.cos_phi.v = m.cos_phi;
       r.tan_phi.v = m.tan_phi;
       r.tan_psi.v = m.tan_psi;
-      r.ic_phi.v = m.ic_phi;
-      r.e_phi.v = m.e_phi;
-      r.n_phi.v = m.n_phi;
     }
     r.bulk.v = m.bulk;
     r.shear.v = m.shear;
