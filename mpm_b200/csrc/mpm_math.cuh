@@ -338,7 +338,7 @@ struct MaterialT {
   // evaluation; softening replaces them per point)
   R sin_phi, cos_phi, tan_phi, tan_psi;
   // and from them 1 / (sqrt(3) cos phi), (3 - sin phi) / (3 + sin phi),
-  // (1 + sin phi) / (1 - sin phi)
+  // (1 + sin phi) / (1 - sin phi): the mixed path's FP32 yield check reads them
   R ic_phi, e_phi, n_phi;
 };
 using MaterialParams = MaterialT<double>;
@@ -588,6 +588,9 @@ struct FrictionTrig {
   R ic, e, n;  // friction_quotients
 };
 
+// From the material's table where the state's angles are the material's: the FP32
+// yield check of every particle.  A mixed return's FP64 angles are the FP32 state's
+// and differ from the FP64 material's, so it evaluates the functions.
 template <typename R>
 MPM_HD FrictionTrig<R> friction_trig(const MaterialT<R>& m, const R* sv) {
   FrictionTrig<R> t;

@@ -13,7 +13,10 @@
 // update.  Each heavy piece is inlined once, everything can stay in
 // registers, and the lanes of a warp that are in different phases run the
 // same pass code together.  Per point the evaluations and their inputs are those
-// of mc_stress<R, PD, false>, so the results are the same bits.
+// of mc_stress<R, PD, false>: the same bits in the units that never fuse a multiply
+// and an add.  In the mixed unit the compiler may fuse differently in different
+// bodies; that the return kernel and the persistent step, which both inline this
+// loop, agree bit for bit is held by a test of flowing columns.
 #pragma once
 
 #include "mpm_math.cuh"
