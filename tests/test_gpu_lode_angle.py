@@ -1,6 +1,6 @@
-"""The Lode angle of the MohrCoulomb update, which the device takes from the triple-angle
-equation: on the triaxial corners (compression, extension), at growing distances from
-them and in between, against 80-bit arithmetic."""
+"""The Lode angle and the other invariants of the MohrCoulomb update as the FP64 path takes them on
+the device (acos of cos 3 theta): on the triaxial corners (compression, extension), at
+growing distances from them and in between, against 80-bit arithmetic."""
 import numpy as np
 import pytest
 
