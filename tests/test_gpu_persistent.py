@@ -50,6 +50,28 @@ def test_3d_mohr_coulomb_column_bitwise(vu):
     assert np.any(p["svars"][:, 0] != 0)  # some points returned plastically
 
 
+@pytest.mark.parametrize("dim", [2, 3])
+def test_flowing_column_bitwise(dim):
+    """Most points on the yield surface, in shear and in tension, with dilation: the return's FP64
+    arithmetic in the persistent kernel and in its own must round alike, wherever the compiler
+    fuses a multiply and an add."""
+    if dim == 3:
+        prob = P.column_3d(shape=(24, 10, 12), block=(12, 10, 10), c=500.0, psi=5.0, dt=1e-5)
+    else:
+        prob = P.column_2d(shape=(60, 40), block=(30, 30), dt=1e-5, scheme="usl", material="MohrCoulomb")
+        prob.materials = [(0, "MohrCoulomb2D", P.mohr_coulomb(1e6, 0.3, 1800.0, 30.0, 500.0, 5.0, tension_cutoff=100.0))]
+
+    def spread(s):
+        st = s.read()
+        st["v"] = st["x"] * (np.arange(dim) == 0) * 2.0 - st["x"] * (np.arange(dim) == dim - 1)
+        s.load(st)
+
+    g, p = _both(prob, [1, 40, 160], 8, prepare=spread)
+    _assert_same(g, p, f"{dim}D flowing column")
+    yields = p["svars"][:, 0]
+    assert np.count_nonzero(yields == 1) > len(yields) // 8 and np.count_nonzero(yields == 2) > 20
+
+
 def test_2d_linear_elastic_column_with_gravity_ramp_bitwise():
     prob = P.column_2d(scheme="usl")
     prob.analysis["gravity_ramping_time"] = 2e-4  # 20 steps
