@@ -86,10 +86,14 @@ const char* kernel_name(int kid);
 // the kernels of the counting sort) with a pair of CUDA events on
 // the launching stream and accumulates their elapsed times.
 // The sort is one kernel (a cluster) up to these sizes and five (reset, count,
-// chunk scans, scan add, fill) above.  Measured, a 2D step with one / five: 3,200
-// particles 16.4 / 18.5 us, 8,000 18.5 / 20.6, 16,384 20.5 / 22.6, 32,400 26.6 /
-// 21.0, 65,536 32.8 / 22.6.
-constexpr int64_t SORT_SMALL_NP = 16384, SORT_SMALL_CELLS = 65536;
+// chunk scans, scan add, fill) above.  Measured, a step with one / five kernels, in
+// us, by particles (2D, mixed, 8,000 cells): 3,200 18.4 / 18.5, 8,000 18.4 / 18.9,
+// 13,900 19.1 / 20.0, 32,400 26.6 / 21.0, 65,536 32.8 / 22.6.  By cells, of 800
+// particles: 4,000 16.4 / 16.8, 8,000 16.4 / 18.5, 17,000 18.4 / 18.5, 36,000 18.5 /
+// 18.5, 66,000 22.5 / 18.5; of 13,900: 4,000 18.5 / 20.5, 17,000 20.5 / 20.5, 36,000
+// 22.5 / 20.5, 66,000 24.8 / 20.5; FP64 in 3D, 15,000 particles: 15,000 29.6 / 30.8,
+// 31,000 30.7 / 30.7, 61,000 34.8 / 31.0 (eight SMs scan what 148 would).
+constexpr int64_t SORT_SMALL_NP = 16384, SORT_SMALL_CELLS = 16384;
 inline int sort_kernels(const DevState& s) {
   return s.np <= SORT_SMALL_NP && s.ncells <= SORT_SMALL_CELLS ? 1 : 5;
 }

@@ -30,6 +30,22 @@ def test_cluster_sort_equals_the_passes(precision, block):
         assert np.array_equal(a[f], b[f], equal_nan=True), f
 
 
+@pytest.mark.parametrize("height", [234, 235])  # 16,380 and 16,450 cells: the rule's line is 16,384
+def test_both_sides_of_the_cell_line(height):
+    prob = P.column_2d(shape=(70, height), block=(64, 64), scheme="usl", dt=1e-4)
+    launches = []
+    s = P.build_solver(prob, precision="mixed")
+    for n in (1, 1):
+        before = s.launch_count
+        s.step(n)
+        launches.append(s.launch_count - before)
+    # sort, P2G, nodes, G2P
+    assert launches == [4 if height == 234 else 8] * 2
+    o = P.build_solver(prob)
+    o.step(2)
+    assert np.array_equal(s.read()["cell"], o.read()["cell"])
+
+
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
 @pytest.mark.parametrize("scheme", ["usl", "usf", "musl"])
 def test_particles_leaving_a_grid_are_found_or_removed(precision, scheme):
