@@ -208,8 +208,9 @@ int mpm_gpu_step_timed(mpm_gpu_t h, int64_t nsteps, double* elapsed_ms);
 /* Launch shape of the steps (no counterpart in the reference, whose steps
  * are host loops): threads of a P2G cell tile on a tensor-product grid (128
  * or 256), threads of a node-kernel block (128 or 256), blocks per SM of the
- * plastic-return kernel (4, 8 or 16); 0 keeps the built-in default (256 up to
- * 100,000 particles and 128 above, 256, 8).  Results do not depend on it.
+ * plastic-return kernel (4, 8 or 16); 0 keeps the built-in default (256, or 128
+ * above 100,000 particles in a mesh that is not mostly empty; 256; 8).  Results
+ * do not depend on it.
  * mpm_gpu_get_launch_shape writes the three values in use.  mpm_gpu_autotune
  * times each candidate over `steps` steps (at least 3, after 3 untimed ones)
  * of the solver's own state, one field at a time, keeps the fastest, and

@@ -1139,7 +1139,7 @@ void step_impl(const DevState& s, const StepArgs& a, cudaStream_t st, Profiler& 
     auto launch = [&](auto aff) {
       constexpr int AFF = decltype(aff)::value;
       constexpr int TT = p2g_tile_t<BOX, AFF>();
-      if (BOX && !AFF && tile_threads(a, BOX, np) == 128)
+      if (BOX && !AFF && tile_threads(a, BOX, DIM, s, false) == 128)
         launch_kernel(!a.returns_first, k_p2g_tiles<DIM, MODE, BOX, AFF, 128>, nblocks(s.ncells, 128 / Elem<DIM>::NV), 128, 0, st, s, a.g[0], a.g[1], a.g[2]);
       else
         launch_kernel(!a.returns_first, k_p2g_tiles<DIM, MODE, BOX, AFF>, nblocks(s.ncells, TT / Elem<DIM>::NV), TT, 0, st, s, a.g[0], a.g[1], a.g[2]);

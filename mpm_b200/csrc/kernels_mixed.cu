@@ -1580,7 +1580,7 @@ void step_mixed(const DevState& s, const StepArgs& a, cudaStream_t st, Profiler&
         return;
       }
     }
-    if (BOX && tile_threads(a, BOX, np) == 128)
+    if (BOX && tile_threads(a, BOX, DIM, s, true) == 128)
       launch_kernel(!a.returns_first, k_p2g_tiles_mixed<DIM, MODE, BOX, 128>, nblk(s.ncells, 128 / NV), 128, 0, st, s);
     else
       launch_kernel(!a.returns_first, k_p2g_tiles_mixed<DIM, MODE, BOX>, nblk(s.ncells, p2g_tile_t<BOX>() / NV),

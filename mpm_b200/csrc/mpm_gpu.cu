@@ -2026,7 +2026,10 @@ int mpm_gpu_get_launch_shape(mpm_gpu_t h, int32_t* shape) {
   MPM_GUARD(h)
   if (!shape) throw InvalidArg("null shape");
   const StepArgs a = base_step_args(h);
-  shape[0] = tile_threads(a, h->structured, h->npad);
+  DevState sizes;
+  sizes.np = h->npad;
+  sizes.ncells = h->ncells;
+  shape[0] = tile_threads(a, h->structured, h->dim, sizes, h->mixed);
   shape[1] = node_block(a);
   shape[2] = return_blocks(a);
   MPM_END(h)

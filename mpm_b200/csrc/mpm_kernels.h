@@ -42,15 +42,25 @@ struct StepArgs {
 };
 
 // The launch shape a step uses: the built-in defaults where a field is zero.
-// P2G tile on a grid: 256 threads up to P2G_WIDE_NP particles, 128 above.  A
-// tile's threads wait for its slowest load, so the smaller one is the faster once
-// the grid fills the GPU many times: step of 129k particles 86.9 / 83.2 us (256 /
-// 128), 256k FP64 126 / 118, 0.8M 260 / 248, 1.3M in 2D 184 / 177, 2M 285 / 276;
-// 37k and fewer alike.
+// P2G tile on a grid: 256 threads, or 128 above P2G_WIDE_NP particles where the
+// mesh is not mostly empty.  A tile's threads wait for its slowest load, so the
+// smaller one is the faster once the grid fills the GPU many times; but an empty
+// tile is a block that starts, reads its cell range and leaves, and there are
+// twice as many of the smaller ones.  Step in us (256 / 128 threads):
+//   by particles (3D, 0.29 cells a particle): mixed 64k 34.2 / 35.0, 97k 38.6 / 38.6,
+//     111k 39.2 / 38.0, 176k 48.1 / 46.1, 0.8M 240 / 230, 2M 289 / 282; FP64 64k 43.4 /
+//     45.2, 85k 52.6 / 51.1, 111k 57.4 / 53.4, 256k 144 / 139;
+//   by particles per 128-thread tile, empty ones counted (3D, 1M particles): mixed 118
+//     155 / 157, 62 160 / 157, 31 175 / 171, 15 187 / 195, 8 220 / 271 (262k: 30 59.0 /
+//     60.9, 8 69 / 86; a footing of 335k: 34 63.9 / 65.1, of 1.6M: 33 230 / 234; 2D,
+//     360k: 62 49.0 / 47.7, 31 52.8 / 53.7); FP64 15 350 / 339, 8 400 / 395 (262k: 15
+//     109 / 108, 8 120 / 126; 2D: 15 95.6 / 96.4).
 constexpr int64_t P2G_WIDE_NP = 100000;
-inline int tile_threads(const StepArgs& a, bool box, int64_t np) {
+inline int tile_threads(const StepArgs& a, bool box, int dim, const DevState& s, bool mixed) {
   if (!box) return 128;
-  return a.p2g_tile ? a.p2g_tile : (np <= P2G_WIDE_NP ? 256 : 128);
+  if (a.p2g_tile) return a.p2g_tile;
+  const int64_t tiles = (s.ncells * (dim == 2 ? 4 : 8) + 127) / 128;
+  return s.np > P2G_WIDE_NP && s.np >= tiles * (mixed ? 40 : 12) ? 128 : 256;
 }
 inline int node_block(const StepArgs& a) { return a.node_threads ? a.node_threads : 256; }
 inline int return_blocks(const StepArgs& a) { return a.return_blocks_per_sm ? a.return_blocks_per_sm : 8; }

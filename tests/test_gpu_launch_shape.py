@@ -69,6 +69,26 @@ def test_autotune_restores_the_state_and_the_run():
     _assert_same(b.read(), ref, "run after autotune")
 
 
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("mesh,tile", [((23, 23, 23), 256),  # 97,336 particles, a full mesh
+                                       ((24, 24, 23), 128),  # 105,984: 128 particles a 128-thread tile
+                                       ((76, 24, 23), 128),  # 40.4 of them, empty tiles counted
+                                       ((77, 24, 23), {"mixed": 256, "fp64": 128}),  # 39.9
+                                       ((255, 24, 23), {"mixed": 256, "fp64": 128}),  # 12.05
+                                       ((257, 24, 23), 256)])
+def test_default_tile_by_particles_and_cells(precision, mesh, tile):
+    """Wide tiles up to 100,000 particles and in sparse meshes; either tile gives the same step."""
+    block = (min(mesh[0], 24), mesh[1], mesh[2])
+    s = P.build_solver(P.column_3d(shape=mesh, block=block, c=500.0), precision=precision)
+    want = tile[precision] if isinstance(tile, dict) else tile
+    assert s.launch_shape()[0] == want, (s.nparticles, mesh)
+    s.step(2)
+    o = P.build_solver(P.column_3d(shape=mesh, block=block, c=500.0), precision=precision)
+    o.set_launch_shape(p2g_tile=384 - want)
+    o.step(2)
+    _assert_same(s.read(), o.read(), mesh)
+
+
 def test_general_mesh_keeps_its_tile():
     from tests.test_gpu_general_mesh import distort_interior
     prob = distort_interior(P.column_2d(shape=(12, 8), block=(4, 6)))
