@@ -72,8 +72,8 @@ BYTES_PER_PARTICLE = {
 # for the roofline's "traffic": the 4M-particle launch is too large for a
 # multi-pass capture.
 MEASURED_TRAFFIC_PER_PARTICLE = {
-    ("mixed", 3): {"g2p": 329.7, "p2g": 117.0},
-    ("fp64", 3): {"g2p": 615.4, "p2g": 186.3},
+    ("mixed", 3): {"g2p": 307.6, "p2g": 97.5},
+    ("fp64", 3): {"g2p": 605.9, "p2g": 176.2},
 }
 # Algorithmic bytes per particle-step of the whole step (compulsory particle-state
 # traffic plus one write and one read of each nodal field per active node), for
