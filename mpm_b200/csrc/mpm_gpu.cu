@@ -1884,9 +1884,13 @@ static int run_steps(mpm_gpu_t h, int64_t nsteps, double* elapsed_ms) {
   // launches).  Every kernel of a step is launched eagerly before a capture of
   // it (the first launch sets shared-memory attributes and loads the kernel):
   // the first step of a call, and of a handle's first call that defers its
-  // returns also the second, which is the first to make any.  Profiling runs
-  // eagerly.
+  // returns also the second, which is the first to make any.  A step whose gravity
+  // is not the step's before (a ramp in progress) is launched eagerly: its graph
+  // would never be replayed, and a capture costs more than a step (800 particles: 240
+  // us a step with the fork of the returns, 135 before it; eagerly 28).  Profiling
+  // runs eagerly.
   bool eager_done = false;
+  double last_g[3] = {0., 0., 0.};
   // Each step's plastic returns run beside the next step's sort; the call's last
   // ones after its last step.
   const bool beside = nsteps > 1 && a.scheme == 1 && h->any_mc && h->ntangent == 0 && !h->prof.enabled;
@@ -1906,10 +1910,12 @@ static int run_steps(mpm_gpu_t h, int64_t nsteps, double* elapsed_ms) {
       gm = std::min(1.0, static_cast<double>(h->step) * h->cfg.dt / h->cfg.gravity_ramping_time);
     for (int d = 0; d < 3; ++d) a.g[d] = d < h->dim ? gm * h->cfg.gravity[d] : 0.;
     const bool graphable = h->graph_ok && !h->prof.enabled && eager_done && (!beside || h->returns_launched);
+    const bool steady = s > 0 && a.g[0] == last_g[0] && a.g[1] == last_g[1] && a.g[2] == last_g[2];
+    for (int d = 0; d < 3; ++d) last_g[d] = a.g[d];
     if (graphable && h->graph && same_step(h->graph_state, h->ds, h->graph_args, a)) {
       ck(cudaGraphLaunch(h->graph, h->stream), "cudaGraphLaunch");
       h->prof.launches += h->graph_launches;
-    } else if (graphable) {
+    } else if (graphable && steady) {
       if (h->graph) cudaGraphExecDestroy(h->graph);
       h->graph = nullptr;
       const int64_t l0 = h->prof.launches;
