@@ -201,8 +201,8 @@ constexpr int tile_min_blocks() {
 
 template <int DIM, int MODE, bool BOX, int AFF, int T = p2g_tile_t<BOX, AFF>()>
 __global__ void __launch_bounds__(T, (tile_min_blocks<BOX, AFF, T>()))
-    k_p2g_tiles(DevState s, double g0, double g1, double g2) {
-  after_previous();
+    k_p2g_tiles(DevState s, double g0, double g1, double g2, bool dependent) {
+  if (dependent) after_previous();
   constexpr int NV = Elem<DIM>::NV;
   constexpr int CB = T / NV;
   constexpr int NVAL = PV<DIM>::N;
@@ -1139,10 +1139,15 @@ void step_impl(const DevState& s, const StepArgs& a, cudaStream_t st, Profiler& 
     auto launch = [&](auto aff) {
       constexpr int AFF = decltype(aff)::value;
       constexpr int TT = p2g_tile_t<BOX, AFF>();
+      auto run = [&](auto kernel, int threads) {
+        const unsigned tiles = nblocks(s.ncells, threads / Elem<DIM>::NV);
+        const bool dependent = p2g_dependent(a, tiles);
+        launch_kernel(dependent, kernel, tiles, threads, 0, st, s, a.g[0], a.g[1], a.g[2], dependent);
+      };
       if (BOX && !AFF && tile_threads(a, BOX, DIM, s, false) == 128)
-        launch_kernel(!a.returns_first, k_p2g_tiles<DIM, MODE, BOX, AFF, 128>, nblocks(s.ncells, 128 / Elem<DIM>::NV), 128, 0, st, s, a.g[0], a.g[1], a.g[2]);
+        run(k_p2g_tiles<DIM, MODE, BOX, AFF, 128>, 128);
       else
-        launch_kernel(!a.returns_first, k_p2g_tiles<DIM, MODE, BOX, AFF>, nblocks(s.ncells, TT / Elem<DIM>::NV), TT, 0, st, s, a.g[0], a.g[1], a.g[2]);
+        run(k_p2g_tiles<DIM, MODE, BOX, AFF>, TT);
     };
     if constexpr (MODE != 1) {  // the mass-momentum mapping velocity
       if (a.vupd == 2 || a.vupd == 4) return launch(std::integral_constant<int, 1>{});
@@ -1300,7 +1305,9 @@ void launch_p2g_nodes_fp64(int dim, const DevState& s, const StepArgs& a, cudaSt
     constexpr int DIM = decltype(dimc)::value;
     constexpr bool BOX = decltype(boxc)::value;
     constexpr int TT = p2g_tile_t<BOX, 0>();
-    launch_dependent(k_p2g_tiles<DIM, 2, BOX, 0>, nblocks(s.ncells, TT / Elem<DIM>::NV), TT, 0, st, s, a.g[0], a.g[1], a.g[2]);
+    const unsigned tiles = nblocks(s.ncells, TT / Elem<DIM>::NV);
+    const bool dependent = p2g_dependent(a, tiles);
+    launch_kernel(dependent, k_p2g_tiles<DIM, 2, BOX, 0>, tiles, TT, 0, st, s, a.g[0], a.g[1], a.g[2], dependent);
     launch_dependent(k_nodes<DIM, 1>, nblocks(s.nn, 256), 256, 0, st, s, a.dt, a.damping);
   };
   if (dim == 2)

@@ -435,8 +435,8 @@ __device__ __forceinline__ void p2g_tile_mixed(const DevState& s, int64_t bx) {
 
 template <int DIM, int MODE, bool BOX, int T = p2g_tile_t<BOX>(), int AFF = 0>
 __global__ void __launch_bounds__(T, (mixed_tile_min_blocks<BOX, T, AFF>()))
-    k_p2g_tiles_mixed(DevState s) {
-  after_previous();
+    k_p2g_tiles_mixed(DevState s, bool dependent) {
+  if (dependent) after_previous();
   p2g_tile_mixed<DIM, MODE, BOX, T, AFF>(s, blockIdx.x);
 }
 
@@ -1569,22 +1569,19 @@ void step_mixed(const DevState& s, const StepArgs& a, cudaStream_t st, Profiler&
   // P2G cell tiles of the step's launch shape
   auto p2g = [&](auto mode) {
     constexpr int MODE = decltype(mode)::value;
-    constexpr int NV = Elem<DIM>::NV;
+    auto launch = [&](auto kernel, int threads) {
+      const unsigned tiles = nblk(s.ncells, threads / Elem<DIM>::NV);
+      const bool dependent = p2g_dependent(a, tiles);
+      launch_kernel(dependent, kernel, tiles, threads, 0, st, s, dependent);
+    };
     if constexpr (MODE != 1) {  // the mass-momentum mapping velocity (128-thread tiles)
-      if (a.vupd == 2 || a.vupd == 4) {
-        launch_kernel(!a.returns_first, k_p2g_tiles_mixed<DIM, MODE, BOX, 128, 1>, nblk(s.ncells, 128 / NV), 128, 0, st, s);
-        return;
-      }
-      if (a.vupd == 3) {
-        launch_kernel(!a.returns_first, k_p2g_tiles_mixed<DIM, MODE, BOX, 128, 2>, nblk(s.ncells, 128 / NV), 128, 0, st, s);
-        return;
-      }
+      if (a.vupd == 2 || a.vupd == 4) return launch(k_p2g_tiles_mixed<DIM, MODE, BOX, 128, 1>, 128);
+      if (a.vupd == 3) return launch(k_p2g_tiles_mixed<DIM, MODE, BOX, 128, 2>, 128);
     }
     if (BOX && tile_threads(a, BOX, DIM, s, true) == 128)
-      launch_kernel(!a.returns_first, k_p2g_tiles_mixed<DIM, MODE, BOX, 128>, nblk(s.ncells, 128 / NV), 128, 0, st, s);
+      launch(k_p2g_tiles_mixed<DIM, MODE, BOX, 128>, 128);
     else
-      launch_kernel(!a.returns_first, k_p2g_tiles_mixed<DIM, MODE, BOX>, nblk(s.ncells, p2g_tile_t<BOX>() / NV),
-                       p2g_tile_t<BOX>(), 0, st, s);
+      launch(k_p2g_tiles_mixed<DIM, MODE, BOX>, p2g_tile_t<BOX>());
   };
   // G2P of the mapping-matrix updates (ASFLIP 2, TPIC 3, APIC 4)
   auto g2p_affine = [&](auto stress) {

@@ -17,13 +17,14 @@ namespace mpm_b200 {
 // access to global memory: lets the next grid of the stream be scheduled and
 // waits until the previous one has completed and its writes are visible.  Every
 // thread calls it, so a grid that has completed implies all before it have.
-// Without effect in a plain launch.
+// Without effect on a plain launch's order, but not free in a block
+// that has little else to do (p2g_dependent).
 __device__ __forceinline__ void after_previous() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-// (dependent false: a plain launch, for a kernel that also waits on another stream)
+// (dependent false: a plain launch)
 template <class... P, class... A>
 inline void launch_kernel(bool dependent, void (*kernel)(P...), unsigned grid, unsigned block,
                           size_t smem, cudaStream_t st, const A&... args) {

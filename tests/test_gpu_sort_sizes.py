@@ -30,6 +30,26 @@ def test_cluster_sort_equals_the_passes(precision, block):
         assert np.array_equal(a[f], b[f], equal_nan=True), f
 
 
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("scheme", ["usl", "usf", "musl"])
+def test_both_launches_of_p2g(precision, scheme):
+    """P2G waits for the sort on the device up to 4,096 tiles and is launched after it above:
+    the same run in meshes of 88, 4,095 and 4,098 tiles, the added ones empty."""
+    states = []
+    for height in (80, 3744, 3746):
+        prob = P.column_2d(shape=(70, height), block=(31, 33), scheme=scheme, dt=1e-4)
+        s = P.build_solver(prob, precision=precision)
+        st = s.read()
+        st["v"] = 5.0 * (st["x"] - st["x"].mean(axis=0)) * np.array([1.0, -0.5])
+        s.load(st)
+        s.step(1)
+        s.step(39)
+        states.append(s.read())
+    for b in states[1:]:
+        for f in FIELDS:
+            assert np.array_equal(states[0][f], b[f], equal_nan=True), f
+
+
 @pytest.mark.parametrize("height", [234, 235])  # 16,380 and 16,450 cells: the rule's line is 16,384
 def test_both_sides_of_the_cell_line(height):
     prob = P.column_2d(shape=(70, height), block=(64, 64), scheme="usl", dt=1e-4)
